@@ -185,6 +185,10 @@ def cuda_problem_source(pc):
     sig_bc = "const double* __restrict__ y0, const double* __restrict__ y1, const double* __restrict__ p, const double* __restrict__ th"
     A = "__device__ __forceinline__ void"
 
+    # structural nonzeros of Df, row-major: the condensation skips the others
+    bits = "".join("1" if e else "0" for e in pc.Df_nz.ravel())
+    out.append("__device__ constexpr char cs_df_nz[] = \"%s\";" % bits)
+    out.append("#define CS_DF_NZ(e) (cs_df_nz[e] == '1')")
     out.append("%s cs_f(%s, double* __restrict__ f) {" % (A, sig_pt))
     out += _cuda_body(pc.f, ["f[%d]" % i for i in range(ny)], pr) if ny else []
     out.append("}")

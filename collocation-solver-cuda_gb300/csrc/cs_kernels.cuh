@@ -128,6 +128,7 @@ struct CsBatch {
   double* wsp;              // [wsp_ctas][wsp_stride]
   long long wsp_stride;     // doubles per CTA
   int wsp_ctas, wsp_pad;
+  unsigned char* zform;     // [T] register condensation: 1 if the z rows of X hold g_z^-1 [g_y g_p g] (0: the solution)
 };
 
 // Large-system kernels (global-memory slab per CTA): CS_BIG_COND selects
@@ -582,6 +583,11 @@ extern "C" __global__ void k_lists(CsBatch bt, int mode, int nlvl) {
 //   X0    [NY+NZ][NRHS]            stage-0 rows of X = W^-1 [J V f_a]
 //   inv   [S1]                     reciprocal pivots
 //   red   [16]                     cross-warp pivot search (CTA groups)
+// structural nonzeros of Df ([NY][NFG], row-major); all, where the problem
+// functions come without them
+#ifndef CS_DF_NZ
+#define CS_DF_NZ(e) true
+#endif
 #define CS_RB (CS_NY + CS_NZ)
 #define CS_S1 ((CS_M - 1) * CS_RB)
 #define CS_NCOL1 (CS_S1 + CS_NRHS)
@@ -838,6 +844,520 @@ __device__ void cs_condense_group(const CsBatch& bt, int slot, bool active, doub
   if (singular && tid == 0) atomicAdd(&bt.inst[b].singular, 1);
 }
 
+// ------------------------------------------------------------------------
+// Register condensation (CS_ZREG): the algebraic unknowns leave first, stage
+// by stage, and the remaining system of the stages 1..M-1 lives in registers.
+//
+//   per stage j:  [Gy Gp gq] = g_z^-1 [g_y g_p g]                (nz x nz)
+//                 [F  P  q ] = [f_y f_p f-y'] - f_z [Gy Gp gq]
+//   reduced:      F_j h sum_k a_jk x_k - x_j = [F P q]_j         (x: y' rows)
+//   stage 0:      x_0 = -[F P q]_0                               (a_0k = 0)
+//
+// so partial-pivot LU runs on (M-1) NY rows instead of (M-1)(NY+NZ): 0.50 of
+// the flops at NY = 4, NZ = 1.  A group of CS_CL lanes condenses an interval;
+// a lane owns whole columns of the augmented matrix (CS_CUS of the unknowns,
+// CS_CRS of the right-hand sides, rows in registers), so the pivot search and
+// the row swaps are register selects and only the multipliers travel (shuffles).
+// What bounds it is the SM's FP64 unit: it takes a warp instruction every ~19
+// cycles whatever its active lanes, which leaves ~70 issue slots per FP64
+// instruction free for the selects, shuffles and addressing.  Fewer lanes per
+// interval leave fewer of them idle in the triangular loops but need more
+// registers: CS_CL is the cheapest of 4, 8, 16, 32 lanes (cs_c_cost) within 84
+// doubles per lane.  Before, the elimination went through shared memory in
+// loops over (row, column) pairs: a division, two loads and a store per FMA,
+// in sequence.  Measured (Van der Pol, all intervals of a batch, GB300): m = 3,
+// 2.15 M intervals 11.25 -> 5.38 ms; m = 4, 266 k 2.74 -> 1.37 ms (85 FP64 warp
+// instructions per interval, the FP64 unit 86 % busy); m = 5, 1.05 M
+// 22.2 -> 9.99 ms.
+//
+// The pivot row is scaled instead of the pivot column (unit upper factor):
+// CS_CUS + CS_CRS multiplications per step instead of one per row.
+//
+// Not every stage system may lose its z unknowns first: with g_z close to
+// singular (an active smoothed constraint), partial pivoting over the whole
+// stage system is what keeps the rounding errors small.  An interval keeps
+// the reduced form only while every entry of F is below 2^5 / h or 2^5 times
+// the largest of f_y (so elimination grew the rows by that much at most, over
+// their unit diagonal or their own entries) and no pivot of g_z is below 10
+// eps; the others are condensed by cs_condense_group, a warp each, after the
+// group pass.
+#define CS_SY ((CS_M - 1) * CS_NY)
+__host__ __device__ constexpr int cs_c_us(int L) { return (CS_SY + L - 1) / L; }
+// one right-hand side too many for whole slots (f_a, the last): its rows are
+// dealt out over the lanes of the group instead (a slot of its own would use
+// one lane in L)
+__host__ __device__ constexpr bool cs_c_split(int L) { return CS_NRHS > L && CS_NRHS % L == 1; }
+__host__ __device__ constexpr int cs_c_rs(int L) { return cs_c_split(L) ? CS_NRHS / L : (CS_NRHS + L - 1) / L; }
+__host__ __device__ constexpr int cs_c_ss(int L) { return cs_c_split(L) ? (CS_SY + L - 1) / L : 0; }
+// FP64 warp instructions per warp of 32 / L intervals: LU, back substitution,
+// fill, and about 150 for the stage functions of L stages
+__host__ __device__ constexpr long cs_c_cost(int L) {
+  long n = 0;
+  for (int k = 0; k < CS_SY; ++k) {
+    int active = cs_c_rs(L);
+    for (int s = 0; s < cs_c_us(L); ++s)
+      if ((s + 1) * L - 1 > k) ++active;
+    n += (long)(CS_SY - 1 - k) * active + active + (long)(CS_SY - 1 - k) * cs_c_rs(L) + 4;
+    if (cs_c_split(L)) n += 2 * ((CS_SY - 1 - k + L - 1) / L) + 1;
+  }
+  n += (long)CS_SY * cs_c_us(L) + (long)(CS_SY * cs_c_rs(L) + cs_c_ss(L)) * (CS_NY + 1);
+  n += 150L * ((CS_M + L - 1) / L);
+  return n * 1000 / (32 / L);
+}
+__host__ __device__ constexpr bool cs_c_fits(int L) { return (cs_c_us(L) + cs_c_rs(L)) * CS_SY + cs_c_ss(L) <= 84; }
+__host__ __device__ constexpr int cs_c_lanes() {
+  int best = 0;
+  for (int L = 4; L <= 32; L *= 2)
+    if (cs_c_fits(L) && (best == 0 || cs_c_cost(L) < cs_c_cost(best))) best = L;
+  return best;
+}
+#if !CS_BIG_COND
+#define CS_CL (CS_SY <= 28 && CS_NZ * (CS_NZ + CS_NRHS) <= 80 ? cs_c_lanes() : 0)
+#else
+#define CS_CL 0
+#endif
+// shared memory of a group (doubles): FQ [M][NY][NRHS], GQ [M][NZ][NRHS], hA [M][M], fb [NY], fx [SY]
+#define CS_CGRP (CS_M * (CS_NY + CS_NZ) * CS_NRHS + CS_M * CS_M + CS_NY + CS_SY)
+
+#if !CS_BIG_COND
+__device__ __noinline__ void cs_condense_pivoted(const CsBatch& bt, int slot, bool active, double* Wm) {
+  cs_condense_group<32>(bt, slot, active, Wm, nullptr);
+}
+
+// -x as an integer operation (the compiler spends an FP64 add on it)
+__device__ __forceinline__ double cs_neg(double x) {
+  return __hiloint2double(__double2hiint(x) ^ (int)0x80000000, __double2loint(x));
+}
+
+// 1 / p to the last bit or two: the reciprocal of the leading 23 bits in FP32,
+// then one third-order step r (1 + e + e^2), e = 1 - p r, |e| < 2^-22 (the
+// truncated geometric series for 1 / (1 - e)): 3 FP64 instructions where the
+// division takes about 9, on the unit that bounds this kernel.  Exponents
+// near the ends of the range (and 0, inf, NaN) divide.
+__device__ __forceinline__ double cs_rcp(double p) {
+  const int hi = __double2hiint(p), lo = __double2loint(p);
+  const int ex = (hi >> 20) & 0x7ff;
+  if (ex < 16 || ex > 2030) return 1.0 / p;
+  // mantissa in [1, 2) as FP32, its reciprocal in (1/2, 1]
+  const unsigned rf = __float_as_uint(__frcp_rn(__uint_as_float(0x3f800000u | ((unsigned)(hi & 0xfffff) << 3) | ((unsigned)lo >> 29))));
+  // the FP32 number as FP64 bits, scaled by 2^(1023 - ex), with p's sign
+  const int rex = (int)(rf >> 23) - 127 + 1023 + (1023 - ex);
+  const double r = __hiloint2double((hi & 0x80000000) | (rex << 20) | (int)((rf >> 3) & 0xfffff), (int)(rf << 29));
+  const double e = fma(-p, r, 1.0);
+  return fma(r, fma(e, e, e), r);
+}
+
+#if CS_NZ > 0
+// A = [g_z | rest] -> rest := g_z^-1 rest, partial pivoting, in registers;
+// true when a pivot is below 10 eps
+template <int k>
+__device__ __forceinline__ bool cs_gauss_jordan(double (&A)[CS_NZ][CS_NZ + CS_NRHS]) {
+  unsigned long long best = cs_abskey(A[k][k]);
+  int pr = k;
+#pragma unroll
+  for (int r = k + 1; r < CS_NZ; ++r) {
+    const unsigned long long v = cs_abskey(A[r][k]);
+    if (v > best) { best = v; pr = r; }
+  }
+#pragma unroll
+  for (int q = k; q < CS_NZ + CS_NRHS; ++q) {
+    const double old = A[k][q];
+    double top = old;
+#pragma unroll
+    for (int r = k + 1; r < CS_NZ; ++r) {
+      const double t = A[r][q];
+      top = (r == pr) ? t : top;
+      A[r][q] = (r == pr) ? old : t;
+    }
+    A[k][q] = top;
+  }
+  const double ip = cs_rcp(A[k][k]);
+#pragma unroll
+  for (int q = k + 1; q < CS_NZ + CS_NRHS; ++q) A[k][q] *= ip;
+#pragma unroll
+  for (int r = 0; r < CS_NZ; ++r)
+    if (r != k) {
+#pragma unroll
+      for (int q = k + 1; q < CS_NZ + CS_NRHS; ++q) A[r][q] = fma(-A[r][k], A[k][q], A[r][q]);
+    }
+  bool bad = best < 0x3ce4000000000000ull;  // 10 * 2^-52
+  if constexpr (k + 1 < CS_NZ) bad |= cs_gauss_jordan<k + 1>(A);
+  return bad;
+}
+#endif
+
+// stage j of one interval: [F P q] and [Gy Gp gq] into shared memory.
+// Returns true when the reduced form is not to be used (see above).
+__device__ __forceinline__ bool cs_stage_reduced(const CsBatch& bt, int slot, int b, int j, double h, const double* hA,
+                                                 double* FQ, double* GQ) {
+  const double* th = bt.th + (size_t)b * (CS_NTH > 0 ? CS_NTH : 1);
+  const double* yi = bt.y + (size_t)slot * CS_NY;
+  const double* yd = bt.ydot + (size_t)slot * CS_M * CS_NY;
+  double pl[CS_NP > 0 ? CS_NP : 1];
+  for (int k = 0; k < CS_NP; ++k) pl[k] = bt.p[(size_t)b * CS_NP + k];
+  double yt[CS_NY], zl[CS_NZ > 0 ? CS_NZ : 1];
+#pragma unroll
+  for (int k = 0; k < CS_NY; ++k) yt[k] = yi[k];
+#pragma unroll
+  for (int q = 0; q < CS_M; ++q) {
+    const double a = hA[j * CS_M + q];
+#pragma unroll
+    for (int k = 0; k < CS_NY; ++k) yt[k] = fma(a, yd[q * CS_NY + k], yt[k]);
+  }
+  for (int k = 0; k < CS_NZ; ++k) zl[k] = bt.zt[((size_t)slot * CS_M + j) * CS_NZ + k];
+  double f[CS_NY], Df[CS_NY * CS_NFG];
+  cs_f(yt, zl, pl, th, f);
+  cs_Df(yt, zl, pl, th, Df);
+#pragma unroll
+  for (int a = 0; a < CS_NY; ++a) f[a] -= yd[j * CS_NY + a];
+  bool bad = false;
+#if CS_NZ > 0
+  // [g_z | g_y g_p g]
+  double A[CS_NZ][CS_NZ + CS_NRHS];
+  {
+    double g[CS_NZ], Dg[CS_NZ * CS_NFG];
+    cs_g(yt, zl, pl, th, bt.inst[b].alpha, g);
+    cs_Dg(yt, zl, pl, th, bt.inst[b].alpha, Dg);
+#pragma unroll
+    for (int a = 0; a < CS_NZ; ++a) {
+#pragma unroll
+      for (int q = 0; q < CS_NZ; ++q) A[a][q] = Dg[a * CS_NFG + CS_NY + q];
+#pragma unroll
+      for (int q = 0; q < CS_NY; ++q) A[a][CS_NZ + q] = Dg[a * CS_NFG + q];
+#pragma unroll
+      for (int q = 0; q < CS_NPE; ++q) A[a][CS_NZ + CS_NY + q] = Dg[a * CS_NFG + CS_NY + CS_NZ + q];
+      A[a][CS_NZ + CS_NRHS - 1] = g[a];
+    }
+  }
+  bad = cs_gauss_jordan<0>(A);
+#pragma unroll
+  for (int a = 0; a < CS_NZ; ++a)
+#pragma unroll
+    for (int q = 0; q < CS_NRHS; ++q) GQ[(j * CS_NZ + a) * CS_NRHS + q] = A[a][CS_NZ + q];
+  // F against f_y and 1 / h, by the exponents
+  int ey = 0, ef = 0;
+#endif
+#pragma unroll
+  for (int a = 0; a < CS_NY; ++a)
+#pragma unroll
+    for (int q = 0; q < CS_NRHS; ++q) {
+      double v = (q < CS_NY) ? Df[a * CS_NFG + q] : ((q < CS_NY + CS_NPE) ? Df[a * CS_NFG + CS_NZ + q] : f[a]);
+#if CS_NZ > 0
+      if (q < CS_NY) ey = max(ey, __double2hiint(v) & 0x7ff00000);
+#pragma unroll
+      for (int e = 0; e < CS_NZ; ++e)
+        if (CS_DF_NZ(a * CS_NFG + CS_NY + e)) v = fma(-Df[a * CS_NFG + CS_NY + e], A[e][CS_NZ + q], v);
+      ef = max(ef, (q < CS_NY) ? __double2hiint(v) & 0x7ff00000 : 0);
+#endif
+      FQ[(j * CS_NY + a) * CS_NRHS + q] = v;
+    }
+#if CS_NZ > 0
+  ef >>= 20;
+  bad |= ef == 0x7ff || (ef > (ey >> 20) + 4 && ef + (int)((__double2hiint(h) >> 20) & 0x7ff) > 2 * 1023 + 4);
+#endif
+  return bad;
+}
+
+// f(CsInt<I>()) for I in [A, B): loops whose bodies need constant indices
+template <int I>
+struct CsInt {
+  static constexpr int value = I;
+};
+template <int A, int B, typename F>
+__device__ __forceinline__ void cs_static_for(F&& f) {
+  if constexpr (A < B) {
+    f(CsInt<A>());
+    cs_static_for<A + 1, B>(f);
+  }
+}
+
+// A group's augmented matrix in registers: column s L + c of the unknowns in
+// U[s] and of the right-hand sides in R[s] of lane c, and (cs_c_split) row
+// i L + c of the last right-hand side in S[i].
+template <int L>
+struct CsReg {
+  double U[cs_c_us(L)][CS_SY];
+  double R[cs_c_rs(L)][CS_SY];
+  double S[cs_c_ss(L) > 0 ? cs_c_ss(L) : 1];
+};
+
+// rows k and pr (k <= pr) of a column in registers change places
+template <int k>
+__device__ __forceinline__ void cs_reg_swap(double (&col)[CS_SY], int pr) {
+  const double old = col[k];
+  double top = old;
+  cs_static_for<k + 1, CS_SY>([&](auto rc) {
+    constexpr int r = decltype(rc)::value;
+    const double t = col[r];
+    top = (r == pr) ? t : top;
+    col[r] = (r == pr) ? old : t;
+  });
+  col[k] = top;
+}
+
+// step k of the LU (a template per step: every register index is static),
+// partial pivoting: largest |entry| of column k, the first on ties
+template <int L, int k>
+__device__ __forceinline__ void cs_reg_lu(CsReg<L>& m, int gi, int c, bool& singular) {
+  constexpr int US = cs_c_us(L), RS = cs_c_rs(L), SS = cs_c_ss(L), SY = CS_SY, ks = k / L;
+  const unsigned full = 0xffffffffu;
+  const int src = gi * L + (k & (L - 1));  // the lane that owns column k
+  unsigned long long best = cs_abskey(m.U[ks][k]);
+  int pr = k;
+  cs_static_for<k + 1, SY>([&](auto rc) {
+    constexpr int r = decltype(rc)::value;
+    const unsigned long long v = cs_abskey(m.U[ks][r]);
+    if (v > best) { best = v; pr = r; }
+  });
+  pr = __shfl_sync(full, pr, src);
+  if (__any_sync(full, pr != k)) {
+    cs_static_for<ks, US>([&](auto sc) { cs_reg_swap<k>(m.U[decltype(sc)::value], pr); });
+    cs_static_for<0, RS>([&](auto sc) { cs_reg_swap<k>(m.R[decltype(sc)::value], pr); });
+    if constexpr (SS > 0) {
+      double pick = m.S[0];
+      cs_static_for<1, SS>([&](auto ic) { pick = (pr / L == decltype(ic)::value) ? m.S[decltype(ic)::value] : pick; });
+      const double vp = __shfl_sync(full, pick, gi * L + (pr & (L - 1)));
+      const double vk = __shfl_sync(full, m.S[ks], src);
+      cs_static_for<ks, SS>([&](auto ic) {
+        constexpr int i = decltype(ic)::value;
+        m.S[i] = (pr == i * L + c) ? vk : m.S[i];
+      });
+      m.S[ks] = (c == (k & (L - 1))) ? vp : m.S[ks];
+    }
+  }
+  const double pv = __shfl_sync(full, m.U[ks][k], src);
+  const bool tiny = cs_abskey(pv) < 0x3ce4000000000000ull;  // bits of 10 * 2^-52 = 2.22e-15
+  singular |= tiny;
+  const double ip = cs_rcp(pv);
+  // pivot row scaled (columns right of k), then the rows below (the columns up
+  // to k take part: what becomes of their rows from k on is not used any
+  // more; a tiny pivot's column stays uneliminated, as the reference leaves it)
+  cs_static_for<(k + 1) / L, US>([&](auto sc) { m.U[decltype(sc)::value][k] *= ip; });
+  cs_static_for<0, RS>([&](auto sc) { m.R[decltype(sc)::value][k] *= ip; });
+  double sk = 0.0;
+  if constexpr (SS > 0) {
+    sk = __shfl_sync(full, m.S[ks], src) * ip;
+    m.S[ks] = (c == (k & (L - 1))) ? sk : m.S[ks];
+  }
+  double mine = 0.0;  // the multiplier of this lane's row of S
+  cs_static_for<k + 1, SY>([&](auto rc) {
+    constexpr int r = decltype(rc)::value;
+    double l = __shfl_sync(full, m.U[ks][r], src);
+    l = tiny ? 0.0 : l;
+    cs_static_for<(k + 1) / L, US>([&](auto sc) {
+      constexpr int s = decltype(sc)::value;
+      m.U[s][r] = fma(-l, m.U[s][k], m.U[s][r]);
+    });
+    cs_static_for<0, RS>([&](auto sc) {
+      constexpr int s = decltype(sc)::value;
+      m.R[s][r] = fma(-l, m.R[s][k], m.R[s][r]);
+    });
+    if constexpr (SS > 0) {
+      mine = (c == r % L) ? l : mine;
+      if constexpr (r % L == L - 1 || r == SY - 1) {
+        m.S[r / L] = fma(-mine, sk, m.S[r / L]);
+        mine = 0.0;
+      }
+    }
+  });
+  if constexpr (k + 1 < SY) cs_reg_lu<L, k + 1>(m, gi, c, singular);
+}
+
+// back substitution with the unit upper factor, rows r .. 1
+template <int L, int r>
+__device__ __forceinline__ void cs_reg_back(CsReg<L>& m, int gi, int c) {
+  if constexpr (r > 0) {
+    constexpr int SS = cs_c_ss(L);
+    const unsigned full = 0xffffffffu;
+    const int src = gi * L + (r & (L - 1));
+    double sr = 0.0;
+    if constexpr (SS > 0) sr = __shfl_sync(full, m.S[r / L], src);
+    double mine = 0.0;
+    cs_static_for<0, r>([&](auto qc) {
+      constexpr int q = decltype(qc)::value;
+      const double u = __shfl_sync(full, m.U[r / L][q], src);
+      cs_static_for<0, cs_c_rs(L)>([&](auto sc) {
+        constexpr int s = decltype(sc)::value;
+        m.R[s][q] = fma(-u, m.R[s][r], m.R[s][q]);
+      });
+      if constexpr (SS > 0) {
+        mine = (c == q % L) ? u : mine;
+        if constexpr (q % L == L - 1 || q == r - 1) {
+          m.S[q / L] = fma(-mine, sr, m.S[q / L]);
+          mine = 0.0;
+        }
+      }
+    });
+    cs_reg_back<L, r - 1>(m, gi, c);
+  }
+}
+
+// the intervals base .. base + 32 / L - 1 of the work list, one warp
+template <int L>
+__device__ __forceinline__ void cs_condense_regs(const CsBatch& bt, long long base, long long total, int njac,
+                                                 double* warp_smem) {
+  constexpr int G = 32 / L, US = cs_c_us(L), RS = cs_c_rs(L), SS = cs_c_ss(L), SY = CS_SY;
+  const int lane = threadIdx.x & 31, gi = lane / L, c = lane & (L - 1);
+  const unsigned full = 0xffffffffu;
+  double* FQ = warp_smem + (size_t)gi * CS_CGRP;
+  double* GQ = FQ + CS_M * CS_NY * CS_NRHS;
+  double* hA = GQ + CS_M * CS_NZ * CS_NRHS;
+  double* fb = hA + CS_M * CS_M;
+  double* fx = fb + CS_NY;
+  const bool active = base + gi < total;
+  const long long it = active ? base + gi : total - 1;
+  const int kq = cs_find(bt.jac_pre, njac, it);
+  const int b = bt.jac[kq];
+  const int slot = bt.off[b] + (int)(it - bt.jac_pre[kq]);
+  const double h = bt.t[slot + 1] - bt.t[slot];
+  for (int e = c; e < CS_M * CS_M; e += L) hA[e] = h * CS_A[e];
+  {
+    const double* yi = bt.y + (size_t)slot * CS_NY;
+    const double* yd = bt.ydot + (size_t)slot * CS_M * CS_NY;
+    for (int k = c; k < CS_NY; k += L) {
+      double s = 0.0;
+#pragma unroll
+      for (int j = 0; j < CS_M; ++j) s = fma(CS_B[j], yd[j * CS_NY + k], s);
+      fb[k] = yi[CS_NY + k] - yi[k] - h * s;
+    }
+  }
+  __syncwarp();
+  bool bad = false;
+#pragma unroll 1
+  for (int j = c; j < CS_M; j += L) bad |= cs_stage_reduced(bt, slot, b, j, h, hA, FQ, GQ);
+  __syncwarp();
+  const unsigned bmask = __ballot_sync(full, bad);
+  const bool keep = (bmask & ((L == 32 ? full : ((1u << (L & 31)) - 1u)) << (gi * L))) == 0u;
+  // ---- the reduced system
+  CsReg<L> m;
+  cs_static_for<0, US>([&](auto sc) {
+    constexpr int s = decltype(sc)::value;
+    const int col = s * L + c;
+    const bool ok = col < SY;
+    const int k = ok ? 1 + col / CS_NY : 1, q = ok ? col % CS_NY : 0;
+    cs_static_for<0, SY>([&](auto rc) {
+      constexpr int row = decltype(rc)::value, j = 1 + row / CS_NY;
+      m.U[s][row] = fma(hA[j * CS_M + k], FQ[(CS_NY + row) * CS_NRHS + q], (col == row) ? -1.0 : 0.0);
+    });
+  });
+  cs_static_for<0, RS>([&](auto sc) {
+    constexpr int s = decltype(sc)::value;
+    const int col = min(s * L + c, CS_NRHS - 1);
+    double x0[CS_NY];  // [F P q]_0 = -x_0
+#pragma unroll
+    for (int q = 0; q < CS_NY; ++q) x0[q] = FQ[q * CS_NRHS + col];
+    cs_static_for<0, SY>([&](auto rc) {
+      constexpr int row = decltype(rc)::value, j = 1 + row / CS_NY;
+      const double* Fr = FQ + (CS_NY + row) * CS_NRHS;
+      double w = Fr[0] * x0[0];
+#pragma unroll
+      for (int q = 1; q < CS_NY; ++q) w = fma(Fr[q], x0[q], w);
+      m.R[s][row] = fma(hA[j * CS_M], w, Fr[col]);
+    });
+  });
+  if constexpr (SS > 0) {
+    cs_static_for<0, SS>([&](auto ic) {
+      constexpr int i = decltype(ic)::value;
+      const int row = min(i * L + c, SY - 1);
+      const double* Fr = FQ + (CS_NY + row) * CS_NRHS;
+      double w = Fr[0] * FQ[CS_NRHS - 1];
+#pragma unroll
+      for (int q = 1; q < CS_NY; ++q) w = fma(Fr[q], FQ[q * CS_NRHS + CS_NRHS - 1], w);
+      m.S[i] = fma(hA[(1 + row / CS_NY) * CS_M], w, Fr[CS_NRHS - 1]);
+    });
+  }
+  bool singular = false;
+  cs_reg_lu<L, 0>(m, gi, c, singular);
+  cs_reg_back<L, CS_SY - 1>(m, gi, c);
+  if constexpr (SS > 0) {
+    cs_static_for<0, SS>([&](auto ic) {
+      constexpr int i = decltype(ic)::value;
+      if (i * L + c < SY) fx[i * L + c] = m.S[i];
+    });
+    __syncwarp();
+  }
+  // ---- X (column-major [NRHS][S]) and the condensed block row, a column per lane
+  if (active && keep) {
+    double* X = bt.X + (size_t)slot * CS_NRHS * CS_S;
+    double* row = bt.rows0 + (size_t)slot * CS_ROWSZ;
+    cs_static_for<0, RS>([&](auto sc) {
+      constexpr int s = decltype(sc)::value;
+      const int col = s * L + c;
+      if (col < CS_NRHS) {
+        double* Xc = X + col * CS_S;
+        double d[CS_NY];
+#pragma unroll
+        for (int a = 0; a < CS_NY; ++a) {
+          const double x0 = FQ[a * CS_NRHS + col];  // -x_0
+          Xc[a] = cs_neg(x0);
+          d[a] = -CS_B[0] * x0;
+        }
+        cs_static_for<0, SY>([&](auto rc) {
+          constexpr int r = decltype(rc)::value, j = 1 + r / CS_NY, a = r % CS_NY;
+          const double x = m.R[s][r];
+          Xc[j * CS_RB + a] = x;
+          d[a] = fma(CS_B[j], x, d[a]);
+        });
+#pragma unroll
+        for (int j = 0; j < CS_M; ++j)
+#pragma unroll
+          for (int a = 0; a < CS_NZ; ++a) Xc[j * CS_RB + CS_NY + a] = GQ[(j * CS_NZ + a) * CS_NRHS + col];
+        if (col < CS_NY) {
+#pragma unroll
+          for (int a = 0; a < CS_NY; ++a) {
+            row[col * CS_NY + a] = fma(h, d[a], (a == col) ? -1.0 : 0.0);  // A
+            row[(CS_NY + col) * CS_NY + a] = (a == col) ? 1.0 : 0.0;       // C = I
+          }
+        } else if (col < CS_NY + CS_NPE) {
+#pragma unroll
+          for (int a = 0; a < CS_NY; ++a) row[(CS_NY + col) * CS_NY + a] = h * d[a];  // H
+        } else {
+#pragma unroll
+          for (int a = 0; a < CS_NY; ++a) row[(2 * CS_NY + CS_NPE) * CS_NY + a] = fma(-h, d[a], cs_neg(fb[a]));  // b
+        }
+      }
+    });
+    if constexpr (SS > 0) {
+      // the dealt-out column: lanes over its rows
+      constexpr int col = CS_NRHS - 1;
+      double* Xc = X + col * CS_S;
+      for (int a = c; a < CS_NY; a += L) {
+        const double x0 = FQ[a * CS_NRHS + col];  // -x_0
+        Xc[a] = cs_neg(x0);
+        double d = -CS_B[0] * x0;
+#pragma unroll
+        for (int j = 1; j < CS_M; ++j) {
+          const double x = fx[(j - 1) * CS_NY + a];
+          Xc[j * CS_RB + a] = x;
+          d = fma(CS_B[j], x, d);
+        }
+        row[(2 * CS_NY + CS_NPE) * CS_NY + a] = fma(-h, d, cs_neg(fb[a]));
+      }
+#if CS_NZ > 0
+      for (int e = c; e < CS_M * CS_NZ; e += L)
+        Xc[(e / CS_NZ) * CS_RB + CS_NY + e % CS_NZ] = GQ[e * CS_NRHS + col];
+#endif
+    }
+    if (c == 0) {
+      bt.zform[slot] = 1;
+      if (singular) atomicAdd(&bt.inst[b].singular, 1);
+    }
+  }
+  // ---- the intervals that keep their z unknowns
+  unsigned todo = __ballot_sync(full, active && !keep && c == 0);
+  while (todo) {
+    const int src = __ffs(todo) - 1;
+    todo &= todo - 1;
+    __syncwarp();
+    const int sl = __shfl_sync(full, slot, src);
+    cs_condense_pivoted(bt, sl, true, warp_smem);
+    if (lane == 0) bt.zform[sl] = 0;
+    __syncwarp();
+  }
+  __syncwarp();
+}
+#endif  // !CS_BIG_COND
+
 #if !CS_BIG_COND
 // lanes per condensation group, from the size of the stage system
 #define CS_CGL ((CS_S1 > 48) ? 256 : ((CS_S1 > 16) ? 16 : 8))
@@ -877,15 +1397,59 @@ __device__ __forceinline__ void cs_condense_entry(const CsBatch& bt) {
   }
 }
 
-extern "C" __global__ void k_condense(CsBatch bt) { cs_condense_entry<CS_CGL>(bt); }
+// Warps take the work list in chunks of 32 / CL intervals, CTA-major, so that
+// a short list spreads over the SMs before it doubles up on one (the FP64 unit
+// is the SM's).
+template <int CL>
+__device__ __forceinline__ void cs_condense_warps(const CsBatch& bt) {
+  extern __shared__ double smem[];
+  const int njac = bt.nlist[1];
+  const long long total = bt.jac_pre[njac];
+  constexpr int G = 32 / (CL > 0 ? CL : 1);
+  constexpr int per_warp = (G * CS_CGRP > CS_GRP_DBL) ? G * CS_CGRP : CS_GRP_DBL;
+  double* wsm = smem + (size_t)(threadIdx.x >> 5) * per_warp;
+  const long long stride = (long long)gridDim.x * (blockDim.x >> 5) * G;
+  for (long long base = ((long long)(threadIdx.x >> 5) * gridDim.x + blockIdx.x) * G; base < total; base += stride)
+    cs_condense_regs<CL>(bt, base, total, njac, wsm);
+}
+
+// [0] lanes per interval of the register condensation (0: not used), [1] its
+// shared memory per warp in bytes
+extern "C" __device__ const int cs_cond_info[2] = {
+    CS_CL, 8 * ((CS_CL > 0 && (32 / (CS_CL > 0 ? CS_CL : 1)) * CS_CGRP > CS_GRP_DBL)
+                    ? (32 / (CS_CL > 0 ? CS_CL : 1)) * CS_CGRP : CS_GRP_DBL)};
+
+template <int CL>
+struct CsCond {
+  __device__ static __forceinline__ void run(const CsBatch& bt) { cs_condense_warps<CL>(bt); }
+};
+template <>
+struct CsCond<0> {
+  __device__ static __forceinline__ void run(const CsBatch& bt) { cs_condense_entry<CS_CGL>(bt); }
+};
+
+// CTAs per SM the registers must leave room for: the matrix takes 2 registers
+// per double, and three or four CTAs of four warps hide the dependent chains
+// (pivot, reciprocal, scaling) of one another better than two
+#define CS_CDBL (CS_CL > 0 ? (cs_c_us(CS_CL > 0 ? CS_CL : 1) + cs_c_rs(CS_CL > 0 ? CS_CL : 1)) * CS_SY : 0)
+#define CS_CCTAS (CS_CDBL <= 32 ? 4 : (CS_CDBL <= 56 ? 3 : 2))
+extern "C" __global__ void __launch_bounds__(CS_CL > 0 ? 128 : 256, CS_CL > 0 ? CS_CCTAS : 1) k_condense(CsBatch bt) { CsCond<CS_CL>::run(bt); }
+// the tuner's candidates where the elimination goes through shared memory: 4,
+// 8, 16 or 32 lanes per interval (fewer lanes: more intervals share each warp
+// instruction of the elimination, whose short loops leave fewer lanes idle)
+template <int GL, bool ON>
+struct CsCondAlt {
+  __device__ static __forceinline__ void run(const CsBatch& bt) { cs_condense_entry<GL>(bt); }
+};
+template <int GL>
+struct CsCondAlt<GL, false> {
+  __device__ static __forceinline__ void run(const CsBatch&) {}
+};
 #if CS_S1 <= 48
-// the tuner's candidates: 4, 8, 16 or 32 lanes per interval (fewer lanes:
-// more intervals share each warp instruction of the elimination, whose
-// short loops leave fewer lanes idle)
-extern "C" __global__ void k_condense_l4(CsBatch bt) { cs_condense_entry<4>(bt); }
-extern "C" __global__ void k_condense_l8(CsBatch bt) { cs_condense_entry<8>(bt); }
-extern "C" __global__ void k_condense_l16(CsBatch bt) { cs_condense_entry<16>(bt); }
-extern "C" __global__ void k_condense_l32(CsBatch bt) { cs_condense_entry<32>(bt); }
+extern "C" __global__ void k_condense_l4(CsBatch bt) { CsCondAlt<4, CS_CL == 0>::run(bt); }
+extern "C" __global__ void k_condense_l8(CsBatch bt) { CsCondAlt<8, CS_CL == 0>::run(bt); }
+extern "C" __global__ void k_condense_l16(CsBatch bt) { CsCondAlt<16, CS_CL == 0>::run(bt); }
+extern "C" __global__ void k_condense_l32(CsBatch bt) { CsCondAlt<32, CS_CL == 0>::run(bt); }
 #endif
 #endif  // !CS_BIG_COND
 
@@ -1447,13 +2011,87 @@ extern "C" __global__ void __launch_bounds__(128) k_upper(CsBatch bt, int l_lo) 
 extern "C" __global__ void k_upper(CsBatch bt, int l_lo) {}
 #endif
 
-// Stage steps: dk = -(X_f + X_J dy_i + X_V dp), warp per interval, lanes
-// over stage rows (the reference re-factorises W instead,
-// collocation_solver_parallel_2d_shared.py:1619-1650).
-extern "C" __global__ void k_recover(CsBatch bt) {
+// Stage steps dk = -(X_f + X_J dy_i + X_V dp) (the reference re-factorises W
+// instead, collocation_solver_parallel_2d_shared.py:1619-1650), a warp per
+// CS_RIV intervals.  First the y' rows, lanes over (interval, row); then the z
+// rows, which the register condensation leaves as Z = g_z^-1 [g_y g_p g]:
+// dz_j = -(Z_g + Z_y dy~_j + Z_p dp) at the stage's own step dy~_j = dy_i +
+// h sum_k a_jk dy'_k: one right-hand side here instead of NRHS there.
+#define CS_RIV 8
+extern "C" __global__ void __launch_bounds__(128) k_recover(CsBatch bt) {
+#if !CS_BIG_COND
+  __shared__ double steps[4][CS_RIV * CS_M * CS_NY];
+#endif
   const int wpc = blockDim.x >> 5, w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int njac = bt.nlist[1];
   const long long total = bt.jac_pre[njac];
+#if !CS_BIG_COND
+  if (CS_CL > 0 && blockDim.x <= 128) {
+    double* sd = steps[w];
+    for (long long base = ((long long)w * gridDim.x + blockIdx.x) * CS_RIV; base < total;
+         base += (long long)gridDim.x * wpc * CS_RIV) {
+      // lane i < CS_RIV finds interval base + i; the others take it by shuffle
+      int slot_l = -1, b_l = 0;
+      double h_l = 0.0;
+      if (lane < CS_RIV && base + lane < total) {
+        const int k = cs_find(bt.jac_pre, njac, base + lane);
+        b_l = bt.jac[k];
+        slot_l = bt.off[b_l] + (int)(base + lane - bt.jac_pre[k]);
+        h_l = bt.t[slot_l + 1] - bt.t[slot_l];
+      }
+      for (int e0 = 0; e0 < CS_RIV * CS_M * CS_NY; e0 += 32) {
+        const int e = e0 + lane;
+        const bool in = e < CS_RIV * CS_M * CS_NY;
+        const int i = in ? e / (CS_M * CS_NY) : 0, r = e - i * (CS_M * CS_NY);
+        const int slot = __shfl_sync(0xffffffffu, slot_l, i), b = __shfl_sync(0xffffffffu, b_l, i);
+        if (in && slot >= 0) {
+          const int j = r / CS_NY, a = r - j * CS_NY;
+          const double* X = bt.X + (size_t)slot * CS_NRHS * CS_S + j * CS_RB + a;
+          const double* dyi = bt.dy + (size_t)slot * CS_NY;
+          double v = X[(CS_NY + CS_NPE) * CS_S];
+#pragma unroll
+          for (int q = 0; q < CS_NY; ++q) v = fma(X[q * CS_S], dyi[q], v);
+          for (int q = 0; q < CS_NPE; ++q) v = fma(X[(CS_NY + q) * CS_S], bt.dp[(size_t)b * CS_NP + q], v);
+          sd[e] = -v;
+          bt.dydot[(size_t)slot * CS_M * CS_NY + r] = -v;
+        }
+      }
+      __syncwarp();
+#if CS_NZ > 0
+      for (int e0 = 0; e0 < CS_RIV * CS_M * CS_NZ; e0 += 32) {
+        const int e = e0 + lane;
+        const bool in = e < CS_RIV * CS_M * CS_NZ;
+        const int i = in ? e / (CS_M * CS_NZ) : 0, r = e - i * (CS_M * CS_NZ);
+        const int slot = __shfl_sync(0xffffffffu, slot_l, i), b = __shfl_sync(0xffffffffu, b_l, i);
+        const double h = __shfl_sync(0xffffffffu, h_l, i);
+        if (in && slot >= 0) {
+          const int j = r / CS_NZ, a = r - j * CS_NZ;
+          const double* X = bt.X + (size_t)slot * CS_NRHS * CS_S + j * CS_RB + CS_NY + a;
+          const double* dyi = bt.dy + (size_t)slot * CS_NY;
+          const double* ds = sd + i * CS_M * CS_NY;
+          const bool reduced = bt.zform[slot] != 0;
+          double v = X[(CS_NY + CS_NPE) * CS_S];
+          for (int q = 0; q < CS_NPE; ++q) v = fma(X[(CS_NY + q) * CS_S], bt.dp[(size_t)b * CS_NP + q], v);
+#pragma unroll
+          for (int q = 0; q < CS_NY; ++q) {
+            double d = dyi[q];
+            if (reduced) {
+              double s = 0.0;
+#pragma unroll
+              for (int k = 0; k < CS_M; ++k) s = fma(CS_A[j * CS_M + k], ds[k * CS_NY + q], s);
+              d = fma(h, s, d);
+            }
+            v = fma(X[q * CS_S], d, v);
+          }
+          bt.dzt[(size_t)slot * CS_M * CS_NZ + r] = -v;
+        }
+      }
+      __syncwarp();
+#endif
+    }
+    return;
+  }
+#endif
   for (long long it = (long long)blockIdx.x * wpc + w; it < total; it += (long long)gridDim.x * wpc) {
     const int k = cs_find(bt.jac_pre, njac, it);
     const int b = bt.jac[k];
@@ -1473,12 +2111,11 @@ extern "C" __global__ void k_recover(CsBatch bt) {
 }
 
 #if !CS_BIG_TREE
-// The whole Newton direction of one instance in one CTA: tree levels up,
-// top system, back substitution down, stage recovery, then the line search
-// starts (alpha = 1).  One launch per super-step instead of 2 L + 3, which is
+// The block rows' solve of one instance in one CTA: tree levels up, top
+// system, back substitution down (k_recover follows).  One launch per super-step instead of 2 L + 3, which is
 // what matters when few instances are left; used for batches of small and
 // medium instances (the per-level kernels above serve large single ones).
-extern "C" __global__ void __launch_bounds__(256) k_babd_cta(CsBatch bt, int recover) {
+extern "C" __global__ void __launch_bounds__(256) k_babd_cta(CsBatch bt) {
   extern __shared__ double smem[];
   const int nw = blockDim.x >> 5, w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   double* top = smem;                                  // CS_TLD x (CS_NT + 1)
@@ -1547,28 +2184,13 @@ extern "C" __global__ void __launch_bounds__(256) k_babd_cta(CsBatch bt, int rec
 #endif
       __syncthreads();
     }
-    // ---- stage recovery, warp per interval, lanes over stage rows (or by
-    //      k_recover across the GPU when recover == 0)
-    for (int iv = w; recover && iv < n0; iv += nw) {
-      const int slot = off + iv;
-      const double* X = bt.X + (size_t)slot * CS_NRHS * CS_S;
-      const double* dyi = bt.dy + (size_t)slot * CS_NY;
-      for (int r = lane; r < CS_S; r += 32) {
-        double v = X[(size_t)(CS_NY + CS_NPE) * CS_S + r];
-        for (int q = 0; q < CS_NY; ++q) v = fma(X[(size_t)q * CS_S + r], dyi[q], v);
-        for (int q = 0; q < CS_NPE; ++q) v = fma(X[(size_t)(CS_NY + q) * CS_S + r], dpv[q], v);
-        const int j = r / (CS_NY + CS_NZ), a = r % (CS_NY + CS_NZ);
-        if (a < CS_NY) bt.dydot[((size_t)slot * CS_M + j) * CS_NY + a] = -v;
-        else bt.dzt[((size_t)slot * CS_M + j) * CS_NZ + (a - CS_NY)] = -v;
-      }
-    }
     __syncthreads();
   }
 }
 
 #else
 // not used for large stage systems (the host never launches it)
-extern "C" __global__ void k_babd_cta(CsBatch bt, int recover) {}
+extern "C" __global__ void k_babd_cta(CsBatch bt) {}
 #endif  // !CS_BIG_TREE
 
 #if CS_BIG

@@ -54,6 +54,7 @@ int set_err(int code, const std::string& msg) {
 struct DriverApi {
   decltype(&cuModuleLoadData) moduleLoadData = nullptr;
   decltype(&cuModuleGetFunction) moduleGetFunction = nullptr;
+  decltype(&cuModuleGetGlobal) moduleGetGlobal = nullptr;
   decltype(&cuModuleUnload) moduleUnload = nullptr;
   decltype(&cuLaunchKernel) launchKernel = nullptr;
   decltype(&cuFuncSetAttribute) funcSetAttribute = nullptr;
@@ -141,6 +142,7 @@ struct CsBatchDev {
   double* wsp;
   long long wsp_stride;
   int wsp_ctas, wsp_pad;
+  unsigned char* zform;
 };
 
 static const int CS_MAXLVL = 32;
@@ -202,6 +204,7 @@ int ensure_context() {
   if (!g_drv.ok) {
     CS_TRY(resolve("cuModuleLoadData", (void**)&g_drv.moduleLoadData));
     CS_TRY(resolve("cuModuleGetFunction", (void**)&g_drv.moduleGetFunction));
+    CS_TRY(resolve("cuModuleGetGlobal", (void**)&g_drv.moduleGetGlobal));
     CS_TRY(resolve("cuModuleUnload", (void**)&g_drv.moduleUnload));
     CS_TRY(resolve("cuLaunchKernel", (void**)&g_drv.launchKernel));
     CS_TRY(resolve("cuFuncSetAttribute", (void**)&g_drv.funcSetAttribute));
@@ -344,6 +347,8 @@ struct cs_module {
   // condensation shape tuner
   CUfunction f_cond_l[4] = {nullptr, nullptr, nullptr, nullptr};  // 4, 8, 16, 32 lanes per interval
   size_t grp_bytes = 0;  // shared memory of one interval group (shared-memory kernel)
+  int reg_lanes = 0;     // register condensation: lanes per interval (0: not used for these sizes) and
+  size_t reg_warp_bytes = 0;  // shared memory per warp, as the kernel program says (cs_cond_info)
   int smem_optin = 0;
   int tune_ver = 0;      // bumped when the tuner changes the shape (graphs re-captured)
 };
@@ -374,8 +379,9 @@ static std::string build_source(const cs_module_desc* d, bool big_cond, bool big
 }
 
 static int compile_cubin(const std::string& src, const std::string& cache_dir, std::vector<char>& cubin) {
-  const char* opts[] = {"--gpu-architecture=sm_103a", "-std=c++17", "-lineinfo"};
-  const int nopt = 3;
+  // (default-device: the lambdas of the unrolled loops are device code)
+  const char* opts[] = {"--gpu-architecture=sm_103a", "-std=c++17", "-lineinfo", "--device-as-default-execution-space"};
+  const int nopt = 4;
   int major = 0, minor = 0;
   nvrtcVersion(&major, &minor);
   std::string key_src = src;
@@ -612,6 +618,28 @@ extern "C" int cs_module_load(const cs_module_desc* d, cs_module** out) {
     for (int k = 0; k < 4; ++k)
       if (g_drv.moduleGetFunction(&M->f_cond_l[k], M->mod, names[k]) != CUDA_SUCCESS) M->f_cond_l[k] = nullptr;
   }
+  if (!M->big_cond) {
+    CUdeviceptr gp = 0;
+    size_t gn = 0;
+    int info[2] = {0, 0};
+    if (g_drv.moduleGetGlobal(&gp, &gn, M->mod, "cs_cond_info") != CUDA_SUCCESS || gn != sizeof(info) ||
+        cudaMemcpy(info, (const void*)gp, sizeof(info), cudaMemcpyDeviceToHost) != cudaSuccess) {
+      g_drv.moduleUnload(M->mod);
+      delete M;
+      return set_err(CS_ERR_CUDA, "missing cs_cond_info");
+    }
+    if (info[0] > 0) {
+      M->reg_lanes = info[0];
+      M->reg_warp_bytes = (size_t)info[1];
+      // four warps per CTA, or as many as the shared memory of a CTA holds
+      int w = 4;
+      while (w > 1 && M->reg_warp_bytes * w > (size_t)smem_optin) w >>= 1;
+      M->cgw = info[0];
+      M->condense_block = 32 * w;
+      M->condense_smem = M->reg_warp_bytes * w;
+      M->condense_per_cta = w * (32 / info[0]);
+    }
+  }
   if (M->big_tree && M->prec_tree) {
     struct {
       CUfunction* f;
@@ -684,6 +712,11 @@ extern "C" int cs_module_load(const cs_module_desc* d, cs_module** out) {
     CS_CUDA(cudaDeviceGetAttribute(&smem_sm2, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev));
     int per_sm = std::max<int>(1, (int)((size_t)smem_sm2 / (M->condense_smem + 1024)));
     per_sm = std::min(per_sm, 2048 / M->condense_block);
+    if (M->reg_lanes) {
+      int pr = 0;
+      CS_CU(g_drv.occupancy(&pr, M->f_condense, M->condense_block, M->condense_smem));
+      per_sm = std::max(1, pr);
+    }
     M->condense_grid = M->sms * per_sm;
   }
   *out = M;
@@ -736,7 +769,7 @@ struct cs_batch {
   // per slot (set 0 / set 1 for the arrays a remesh rewrites)
   DBuf t[2], y[2], ydot[2], zt[2], znode[2];
   int cur = 0;
-  DBuf inst_of, dy, dydot, dzt, X, rows0, rows1, tree, res;
+  DBuf inst_of, dy, dydot, dzt, X, rows0, rows1, tree, res, zform;
   // refinement (tensor-core tree): the condensed blocks as condensed, the
   // direction a correction is added to
   DBuf rows_keep, dy_keep, dp_keep;
@@ -825,6 +858,7 @@ static int alloc_slots(cs_batch* bt, long long cap, bool keep_current) {
   CS_TRY(dalloc(bt->rows1, c * M->rowsz * d));
   CS_TRY(dalloc(bt->tree, c * M->treesz * d));
   CS_TRY(dalloc(bt->res, c * d));
+  CS_TRY(dalloc(bt->zform, c));
   if (M->prec_tree) {
     CS_TRY(dalloc(bt->rows_keep, c * M->rowsz * d));
     CS_TRY(dalloc(bt->dy_keep, c * M->ny * d));
@@ -881,6 +915,7 @@ static CsBatchDev devview(cs_batch* bt) {
   v.rows1 = (double*)bt->rows1.p;
   v.tree = (double*)bt->tree.p;
   v.res = (double*)bt->res.p;
+  v.zform = (unsigned char*)bt->zform.p;
   v.znode = (double*)bt->znode[s].p;
   v.inst = (CsInst*)bt->dinst.p;
   v.counters = (unsigned long long*)bt->dcounters.p;
@@ -967,8 +1002,12 @@ static int run_insts(cs_batch* bt, CUfunction f, void** args) { return launch(bt
 static int run_condense(cs_batch* bt, CsBatchDev& v) {
   cs_module* M = bt->M;
   void* args[] = {&v};
-  // intervals per CTA: groups of cgw lanes (shared-memory kernel), one (large systems)
-  const long long per_cta = M->big_cond ? 1 : std::max(1, M->condense_block / std::max(1, M->cgw));
+  // intervals per CTA: groups of cgw lanes (shared-memory kernel), one (large
+  // systems); register condensation: one warp's, since a short list is spread
+  // over the CTAs first
+  const long long per_cta = M->big_cond ? 1
+                            : M->reg_lanes ? 32 / M->reg_lanes
+                                           : std::max(1, M->condense_block / std::max(1, M->cgw));
   return launch_k(bt, M->f_condense, capped(bt, (unsigned)M->condense_grid, 1, per_cta), M->condense_block,
                   M->condense_smem, args, 0);
 }
@@ -1028,8 +1067,7 @@ static int run_lists(cs_batch* bt, CsBatchDev& v, int mode, int nlvl) {
 static int run_direction(cs_batch* bt, CsBatchDev& v, int nlvl) {
   cs_module* M = bt->M;
   if (use_cta_path(bt)) {
-    int recover = 0;
-    void* a[] = {&v, &recover};
+    void* a[] = {&v};
     CS_TRY(launch_k(bt, M->f_babd_cta, (unsigned)(M->sms * 2), 256, M->babd_cta_smem, a, 1));
     void* ar[] = {&v};
     return launch_k(bt, M->f_recover, (unsigned)(M->sms * 8), 128, 0, ar, 1);
@@ -1173,7 +1211,7 @@ extern "C" void cs_batch_free(cs_batch* bt) {
   if (!bt) return;
   if (bt->stream) cudaStreamSynchronize(bt->stream);
   DBuf* all[] = {&bt->dN, &bt->doff, &bt->doff2, &bt->dp, &bt->dth, &bt->ddp, &bt->dinst, &bt->dcounters, &bt->dtrials,
-                 &bt->inst_of, &bt->dy, &bt->dydot, &bt->dzt, &bt->X, &bt->rows0, &bt->rows1, &bt->tree, &bt->res,
+                 &bt->inst_of, &bt->dy, &bt->dydot, &bt->dzt, &bt->X, &bt->rows0, &bt->rows1, &bt->tree, &bt->res, &bt->zform,
                  &bt->iN, &bt->ioff, &bt->it, &bt->iy, &bt->iz, &bt->ip, &bt->l_act, &bt->l_jac, &bt->l_acc,
                  &bt->l_actp, &bt->l_jacp, &bt->l_accp, &bt->l_lvlp, &bt->l_n, &bt->wsp,
                  &bt->rows_keep, &bt->dy_keep, &bt->dp_keep};
@@ -2056,7 +2094,19 @@ extern "C" int cs_autotune_condense(cs_batch* bt, int reps, cs_tune_result* out)
   };
   std::vector<Cand> cands;
   cands.push_back({M->f_condense, M->big_cond ? 0 : M->cgw, M->condense_block, M->condense_grid, M->condense_smem});
-  if (!M->big_cond) {
+  if (!M->big_cond && M->reg_lanes) {
+    // register condensation: warps per CTA
+    for (int w = 1; w <= 4; w *= 2) {
+      const size_t smem = M->reg_warp_bytes * w;
+      if (smem > (size_t)M->smem_optin) break;
+      if (smem > 48 * 1024)
+        CS_CU(g_drv.funcSetAttribute(M->f_condense, CU_FUNC_ATTRIBUTE_MAX_DYNAMIC_SHARED_SIZE_BYTES, (int)smem));
+      int per_sm = 0;
+      CS_CU(g_drv.occupancy(&per_sm, M->f_condense, 32 * w, smem));
+      if (per_sm < 1) continue;
+      cands.push_back({M->f_condense, M->reg_lanes, 32 * w, M->sms * per_sm, smem});
+    }
+  } else if (!M->big_cond) {
     const int lanes[4] = {4, 8, 16, 32};
     for (int k = 0; k < 4; ++k) {
       if (!M->f_cond_l[k]) continue;
