@@ -774,6 +774,7 @@ struct cs_batch {
   // direction a correction is added to
   DBuf rows_keep, dy_keep, dp_keep;
   DBuf wsp;  // large stage systems: slab per CTA
+  CsTextScratch text;  // cs_format_solutions
   std::vector<int> hN, hoff;
   cs_opts opts;
   // work lists
@@ -1216,6 +1217,7 @@ extern "C" void cs_batch_free(cs_batch* bt) {
                  &bt->l_actp, &bt->l_jacp, &bt->l_accp, &bt->l_lvlp, &bt->l_n, &bt->wsp,
                  &bt->rows_keep, &bt->dy_keep, &bt->dp_keep};
   for (DBuf* b : all) dfree(*b);
+  cs_text_scratch_free(&bt->text);
   for (int k = 0; k < 2; ++k)
     if (bt->graph[k]) cudaGraphExecDestroy(bt->graph[k]);
   if (bt->h_n) cudaFreeHost(bt->h_n);
@@ -1692,7 +1694,9 @@ extern "C" int cs_format_solutions(cs_batch* bt, char* out, long long cap, long 
   a.np = M->np;
   a.dN = (const int*)bt->dN.p;
   a.doff = (const int*)bt->doff.p;
+  a.hN = bt->hN.data();
   a.stream = bt->stream;
+  a.scratch = &bt->text;
   bt->launches += 3;
   return cs_text_files(a, out, cap, offsets);
 }
