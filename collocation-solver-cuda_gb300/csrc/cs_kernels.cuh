@@ -167,6 +167,76 @@ __device__ __forceinline__ unsigned long long cs_abs_bits(double v) {
 }
 __device__ __forceinline__ double cs_from_bits(unsigned long long b) { return __longlong_as_double((long long)b); }
 
+// f(CsInt<I>()) for I in [A, B): loops whose bodies need constant indices
+template <int I>
+struct CsInt {
+  static constexpr int value = I;
+};
+template <int A, int B, typename F>
+__device__ __forceinline__ void cs_static_for(F&& f) {
+  if constexpr (A < B) {
+    f(CsInt<A>());
+    cs_static_for<A + 1, B>(f);
+  }
+}
+
+// -x as an integer operation (the compiler spends an FP64 add on it)
+__device__ __forceinline__ double cs_neg(double x) {
+  return __hiloint2double(__double2hiint(x) ^ (int)0x80000000, __double2loint(x));
+}
+
+// 1 / p to the last bit or two: the reciprocal of the leading 23 bits in FP32,
+// then one third-order step r (1 + e + e^2), e = 1 - p r, |e| < 2^-22 (the
+// truncated geometric series for 1 / (1 - e)): 3 FP64 instructions where the
+// division takes about 9, on the unit that bounds these kernels.  Exponents
+// near the ends of the range (and 0, inf, NaN) divide.
+__device__ __forceinline__ double cs_rcp(double p) {
+  const int hi = __double2hiint(p), lo = __double2loint(p);
+  const int ex = (hi >> 20) & 0x7ff;
+  if (ex < 16 || ex > 2030) return 1.0 / p;
+  // mantissa in [1, 2) as FP32, its reciprocal in (1/2, 1]
+  const unsigned rf = __float_as_uint(__frcp_rn(__uint_as_float(0x3f800000u | ((unsigned)(hi & 0xfffff) << 3) | ((unsigned)lo >> 29))));
+  // the FP32 number as FP64 bits, scaled by 2^(1023 - ex), with p's sign
+  const int rex = (int)(rf >> 23) - 127 + 1023 + (1023 - ex);
+  const double r = __hiloint2double((hi & 0x80000000) | (rex << 20) | (int)((rf >> 3) & 0xfffff), (int)(rf << 29));
+  const double e = fma(-p, r, 1.0);
+  return fma(r, fma(e, e, e), r);
+}
+
+// 1 / sqrt(x), x > 0, to the last bit or two: FP32 on the leading bits, then
+// r (1 + h/2 + 3 h^2/8), h = 1 - x r^2, |h| < 2^-20 (the truncated binomial
+// series of (1 - h)^(-1/2)): 5 FP64 instructions in a chain
+__device__ __forceinline__ double cs_rsqrt(double x) {
+  const int hi = __double2hiint(x), lo = __double2loint(x);
+  const int ex = (hi >> 20) & 0x7ff;
+  if (hi < 0 || ex < 16 || ex > 2030) return 1.0 / sqrt(x);
+  const int odd = (ex & 1) ^ 1;  // 1023 is odd: mantissa 2^odd in [1, 4)
+  const float m = __uint_as_float(((unsigned)(127 + odd) << 23) | ((unsigned)(hi & 0xfffff) << 3) | ((unsigned)lo >> 29));
+  const unsigned rf = __float_as_uint(rsqrtf(m));
+  const int rex = (int)(rf >> 23) - 127 + 1023 - ((ex - 1023 - odd) >> 1);
+  const double r = __hiloint2double((rex << 20) | (int)((rf >> 3) & 0xfffff), (int)(rf << 29));
+  const double h = fma(-(x * r), r, 1.0);
+  return fma(r, h * fma(0.375, h, 0.5), r);
+}
+
+// Householder reflector H = I - t v v^T of a column with sum of squares ss and
+// leading entry x0: H column = g e_0 (the sign rule of
+// matrix_factorization_cuda.py:37-54), v_0 = x0 - g, v the column below, and
+// t = 2 / |v|^2 = 1 / (ss + |x0 g|).  False when |v|^2 < eps (nothing to
+// eliminate).  A square root and two divisions before: with few merges in
+// flight their latency (about 600 cycles each) was a third of a merge.
+__device__ __forceinline__ bool cs_reflector(double ss, double x0, double* g, double* v0, double* t) {
+  const double a = ss * cs_rsqrt(ss);
+  const double gg = (__double2hiint(x0) >= 0) ? cs_neg(a) : a;
+  const double half = fma(fabs(x0), a, ss);
+  *g = gg;
+  *v0 = x0 - gg;
+  *t = cs_rcp(half);
+  // half >= eps / 2, as integers (false for NaN)
+  const long long b = __double_as_longlong(half);
+  return b >= 0x3ca0000000000000ll && b <= 0x7ff0000000000000ll;
+}
+
 // Max of non-negative double bit patterns over the lanes of a warp that share
 // an instance, then one atomicMax per instance.  All 32 lanes must call it.
 __device__ __forceinline__ void cs_warp_max_atomic(unsigned long long* dst, int key, unsigned long long v, bool active) {
@@ -924,29 +994,6 @@ __device__ __noinline__ void cs_condense_pivoted(const CsBatch& bt, int slot, bo
   cs_condense_group<32>(bt, slot, active, Wm, nullptr);
 }
 
-// -x as an integer operation (the compiler spends an FP64 add on it)
-__device__ __forceinline__ double cs_neg(double x) {
-  return __hiloint2double(__double2hiint(x) ^ (int)0x80000000, __double2loint(x));
-}
-
-// 1 / p to the last bit or two: the reciprocal of the leading 23 bits in FP32,
-// then one third-order step r (1 + e + e^2), e = 1 - p r, |e| < 2^-22 (the
-// truncated geometric series for 1 / (1 - e)): 3 FP64 instructions where the
-// division takes about 9, on the unit that bounds this kernel.  Exponents
-// near the ends of the range (and 0, inf, NaN) divide.
-__device__ __forceinline__ double cs_rcp(double p) {
-  const int hi = __double2hiint(p), lo = __double2loint(p);
-  const int ex = (hi >> 20) & 0x7ff;
-  if (ex < 16 || ex > 2030) return 1.0 / p;
-  // mantissa in [1, 2) as FP32, its reciprocal in (1/2, 1]
-  const unsigned rf = __float_as_uint(__frcp_rn(__uint_as_float(0x3f800000u | ((unsigned)(hi & 0xfffff) << 3) | ((unsigned)lo >> 29))));
-  // the FP32 number as FP64 bits, scaled by 2^(1023 - ex), with p's sign
-  const int rex = (int)(rf >> 23) - 127 + 1023 + (1023 - ex);
-  const double r = __hiloint2double((hi & 0x80000000) | (rex << 20) | (int)((rf >> 3) & 0xfffff), (int)(rf << 29));
-  const double e = fma(-p, r, 1.0);
-  return fma(r, fma(e, e, e), r);
-}
-
 #if CS_NZ > 0
 // A = [g_z | rest] -> rest := g_z^-1 rest, partial pivoting, in registers;
 // true when a pivot is below 10 eps
@@ -1056,19 +1103,6 @@ __device__ __forceinline__ bool cs_stage_reduced(const CsBatch& bt, int slot, in
   bad |= ef == 0x7ff || (ef > (ey >> 20) + 4 && ef + (int)((__double2hiint(h) >> 20) & 0x7ff) > 2 * 1023 + 4);
 #endif
   return bad;
-}
-
-// f(CsInt<I>()) for I in [A, B): loops whose bodies need constant indices
-template <int I>
-struct CsInt {
-  static constexpr int value = I;
-};
-template <int A, int B, typename F>
-__device__ __forceinline__ void cs_static_for(F&& f) {
-  if constexpr (A < B) {
-    f(CsInt<A>());
-    cs_static_for<A + 1, B>(f);
-  }
 }
 
 // A group's augmented matrix in registers: column s L + c of the unknowns in
@@ -1526,46 +1560,93 @@ __device__ void cs_merge_warp(const double* ra, const double* rb, double* out_ro
 }
 
 // Small blocks (2 NY x QC doubles fit in registers): one thread per merge,
-// fully unrolled, the same Householder steps as cs_merge_warp.
+// fully unrolled.  The sums over the rows run in two chains (rows k, k + 2, ..
+// and k + 1, k + 3, ..): a dependent FP64 instruction waits ~64 cycles.
+// L0 (block rows as condensed): C = I, so the pivot columns start as unit
+// vectors over A_b and stay zero in rows k + 1 .. NY - 1 (no reflector before k
+// reaches them), and before the first reflector the y_l columns are zero below
+// and the y_r columns a unit matrix below: those terms are left out (they add
+// exact zeros), 30 % of the level's FP64 instructions, and C is not read.
+// Measured, level 0 of 2.15 M intervals: 1.55 -> 1.15 ms.
 #define CS_TREE_THREAD (2 * CS_NY * CS_QC <= 128)
 #if CS_TREE_THREAD
+// column c of the merge matrix
+template <bool L0>
+__device__ __forceinline__ void cs_merge_column(const double* __restrict__ ra, const double* __restrict__ rb, int c,
+                                                double (&q)[2 * CS_NY]) {
+#pragma unroll
+  for (int r = 0; r < CS_NY; ++r) {
+    double top = 0.0, bot = 0.0;
+    if (c < CS_NY) { top = L0 ? (r == c ? 1.0 : 0.0) : ra[(CS_NY + c) * CS_NY + r]; bot = rb[c * CS_NY + r]; }
+    else if (c < 2 * CS_NY) { top = ra[(c - CS_NY) * CS_NY + r]; }
+    else if (c < 3 * CS_NY) { bot = L0 ? (r == c - 2 * CS_NY ? 1.0 : 0.0) : rb[(CS_NY + c - 2 * CS_NY) * CS_NY + r]; }
+    else if (c < CS_QC) { top = ra[(2 * CS_NY + c - 3 * CS_NY) * CS_NY + r]; bot = rb[(2 * CS_NY + c - 3 * CS_NY) * CS_NY + r]; }
+    q[r] = top;
+    q[CS_NY + r] = bot;
+  }
+}
+
+// row r is in reflector k
+template <bool L0>
+__device__ __forceinline__ constexpr bool cs_in_reflector(int k, int r) {
+  return r == k || (r > k && !(L0 && r < CS_NY));
+}
+
+// column q (column c of the merge matrix) through the reflector (v below v0, t) of column k
+template <bool L0>
+__device__ __forceinline__ void cs_reflect(int k, int c, double v0, const double (&v)[2 * CS_NY], double t,
+                                           double (&q)[2 * CS_NY]) {
+  const bool low0 = L0 && k == 0 && c >= CS_NY && c < 2 * CS_NY;       // zero below
+  const bool unit0 = L0 && k == 0 && c >= 2 * CS_NY && c < 3 * CS_NY;  // zero above, unit below
+  double w0 = unit0 ? 0.0 : v0 * q[k], w1 = 0.0;
+  if (unit0) {
+#pragma unroll
+    for (int r = CS_NY; r < 2 * CS_NY; ++r)
+      if (r - CS_NY == c - 2 * CS_NY) w0 = v[r];
+  } else if (!low0) {
+    bool first = true;
+#pragma unroll
+    for (int r = k + 1; r < 2 * CS_NY; ++r)
+      if (cs_in_reflector<L0>(k, r)) {
+        if (((r - k) & 1) == 0) w0 = fma(v[r], q[r], w0);
+        else if (first) { w1 = v[r] * q[r]; first = false; }
+        else w1 = fma(v[r], q[r], w1);
+      }
+  }
+  const double bw = -t * (low0 || unit0 ? w0 : w0 + w1);
+  q[k] = unit0 ? bw * v0 : fma(bw, v0, q[k]);
+#pragma unroll
+  for (int r = k + 1; r < 2 * CS_NY; ++r)
+    if (cs_in_reflector<L0>(k, r)) q[r] = low0 ? bw * v[r] : fma(bw, v[r], q[r]);
+}
+
+// sum of squares of column q from row k
+template <bool L0>
+__device__ __forceinline__ double cs_column_ss(int k, const double (&q)[2 * CS_NY]) {
+  double a = q[k] * q[k], b = 0.0;
+  bool first = true;
+#pragma unroll
+  for (int r = k + 1; r < 2 * CS_NY; ++r)
+    if (cs_in_reflector<L0>(k, r)) {
+      if (((r - k) & 1) == 0) a = fma(q[r], q[r], a);
+      else if (first) { b = q[r] * q[r]; first = false; }
+      else b = fma(q[r], q[r], b);
+    }
+  return a + b;
+}
+
+template <bool L0>
 __device__ __forceinline__ void cs_merge_thread(const double* __restrict__ ra, const double* __restrict__ rb,
                                                 double* __restrict__ out_row, double* __restrict__ rec) {
   double Q[CS_QC][2 * CS_NY];
 #pragma unroll
-  for (int c = 0; c < CS_QC; ++c)
-#pragma unroll
-    for (int r = 0; r < CS_NY; ++r) {
-      double top, bot;
-      if (c < CS_NY) { top = ra[(CS_NY + c) * CS_NY + r]; bot = rb[c * CS_NY + r]; }
-      else if (c < 2 * CS_NY) { top = ra[(c - CS_NY) * CS_NY + r]; bot = 0.0; }
-      else if (c < 3 * CS_NY) { top = 0.0; bot = rb[(CS_NY + c - 2 * CS_NY) * CS_NY + r]; }
-      else if (c < 3 * CS_NY + CS_NPE) { top = ra[(2 * CS_NY + c - 3 * CS_NY) * CS_NY + r]; bot = rb[(2 * CS_NY + c - 3 * CS_NY) * CS_NY + r]; }
-      else { top = ra[(2 * CS_NY + CS_NPE) * CS_NY + r]; bot = rb[(2 * CS_NY + CS_NPE) * CS_NY + r]; }
-      Q[c][r] = top;
-      Q[c][CS_NY + r] = bot;
-    }
+  for (int c = 0; c < CS_QC; ++c) cs_merge_column<L0>(ra, rb, c, Q[c]);
 #pragma unroll
   for (int k = 0; k < CS_NY; ++k) {
-    double ss = 0.0;
+    double g, v0, t;
+    if (cs_reflector(cs_column_ss<L0>(k, Q[k]), Q[k][k], &g, &v0, &t)) {
 #pragma unroll
-    for (int r = k; r < 2 * CS_NY; ++r) ss = fma(Q[k][r], Q[k][r], ss);
-    const double x0 = Q[k][k];
-    const double g = (x0 >= 0.0) ? -sqrt(ss) : sqrt(ss);
-    const double v0 = x0 - g;
-    const double vs = ss - x0 * x0 + v0 * v0;
-    if (vs >= CS_EPS) {
-      const double beta = -2.0 / vs;
-#pragma unroll
-      for (int c = k + 1; c < CS_QC; ++c) {
-        double w = v0 * Q[c][k];
-#pragma unroll
-        for (int r = k + 1; r < 2 * CS_NY; ++r) w = fma(Q[k][r], Q[c][r], w);
-        const double bw = beta * w;
-        Q[c][k] = fma(bw, v0, Q[c][k]);
-#pragma unroll
-        for (int r = k + 1; r < 2 * CS_NY; ++r) Q[c][r] = fma(bw, Q[k][r], Q[c][r]);
-      }
+      for (int c = k + 1; c < CS_QC; ++c) cs_reflect<L0>(k, c, v0, Q[k], t, Q[c]);
       Q[k][k] = g;
 #pragma unroll
       for (int r = k + 1; r < 2 * CS_NY; ++r) Q[k][r] = 0.0;
@@ -1582,28 +1663,31 @@ __device__ __forceinline__ void cs_merge_thread(const double* __restrict__ ra, c
   }
 }
 
+// y_m = R^-1 (d - G y_l - E y_r - J p).  The reciprocals of the diagonal leave
+// the chain; an exactly zero diagonal gives a zero component.
 __device__ __forceinline__ void cs_backsub_thread(const double* __restrict__ rec, const double* __restrict__ yl,
                                                   const double* __restrict__ yr, const double* __restrict__ dpv,
                                                   double* __restrict__ ym) {
-  double v[CS_NY];
+  double v[CS_NY], inv[CS_NY];
 #pragma unroll
   for (int a = 0; a < CS_NY; ++a) {
-    double s = rec[(3 * CS_NY + CS_NPE) * CS_NY + a];
+    double s = rec[(3 * CS_NY + CS_NPE) * CS_NY + a], u = rec[(2 * CS_NY) * CS_NY + a] * yr[0];
 #pragma unroll
-    for (int c = 0; c < CS_NY; ++c) s -= rec[(CS_NY + c) * CS_NY + a] * yl[c];
+    for (int c = 0; c < CS_NY; ++c) s = fma(-rec[(CS_NY + c) * CS_NY + a], yl[c], s);
 #pragma unroll
-    for (int c = 0; c < CS_NY; ++c) s -= rec[(2 * CS_NY + c) * CS_NY + a] * yr[c];
+    for (int c = 1; c < CS_NY; ++c) u = fma(rec[(2 * CS_NY + c) * CS_NY + a], yr[c], u);
 #pragma unroll
-    for (int c = 0; c < CS_NPE; ++c) s -= rec[(3 * CS_NY + c) * CS_NY + a] * dpv[c];
-    v[a] = s;
+    for (int c = 0; c < CS_NPE; ++c) u = fma(rec[(3 * CS_NY + c) * CS_NY + a], dpv[c], u);
+    v[a] = s - u;
+    const double d = rec[a * CS_NY + a];
+    inv[a] = cs_abskey(d) != 0ull ? cs_rcp(d) : 0.0;
   }
 #pragma unroll
   for (int r = CS_NY - 1; r >= 0; --r) {
-    const double rr = rec[r * CS_NY + r];
-    const double xr = (rr != 0.0) ? v[r] / rr : 0.0;
+    const double xr = v[r] * inv[r];
     v[r] = xr;
 #pragma unroll
-    for (int a = 0; a < r; ++a) v[a] -= rec[r * CS_NY + a] * xr;
+    for (int a = 0; a < r; ++a) v[a] = fma(-rec[r * CS_NY + a], xr, v[a]);
   }
 #pragma unroll
   for (int a = 0; a < CS_NY; ++a) ym[a] = v[a];
@@ -1620,48 +1704,46 @@ __device__ __forceinline__ void cs_backsub_thread(const double* __restrict__ rec
 // and the SM's FP64 unit takes one warp instruction per ~19 cycles whatever
 // the number of active lanes).
 #define CS_TL ((CS_QC <= 16) ? 16 : 32)
+template <bool L0>
 __device__ __forceinline__ void cs_merge_lanes(const double* __restrict__ ra, const double* __restrict__ rb,
                                                double* __restrict__ out_row, double* __restrict__ rec, bool active) {
   const int c = threadIdx.x & (CS_TL - 1);
   // the group's own lanes: two groups of a warp may take different branches
   const unsigned gm = (CS_TL == 32) ? 0xffffffffu : (0xffffu << (threadIdx.x & 16));
   double Q[2 * CS_NY];
-#pragma unroll
-  for (int r = 0; r < CS_NY; ++r) {
-    double top = 0.0, bot = 0.0;
-    if (c < CS_NY) { top = ra[(CS_NY + c) * CS_NY + r]; bot = rb[c * CS_NY + r]; }
-    else if (c < 2 * CS_NY) { top = ra[(c - CS_NY) * CS_NY + r]; }
-    else if (c < 3 * CS_NY) { bot = rb[(CS_NY + c - 2 * CS_NY) * CS_NY + r]; }
-    else if (c < 3 * CS_NY + CS_NPE) { top = ra[(2 * CS_NY + c - 3 * CS_NY) * CS_NY + r]; bot = rb[(2 * CS_NY + c - 3 * CS_NY) * CS_NY + r]; }
-    else if (c < CS_QC) { top = ra[(2 * CS_NY + CS_NPE) * CS_NY + r]; bot = rb[(2 * CS_NY + CS_NPE) * CS_NY + r]; }
-    Q[r] = top;
-    Q[CS_NY + r] = bot;
-  }
+  cs_merge_column<L0>(ra, rb, c, Q);
 #pragma unroll
   for (int k = 0; k < CS_NY; ++k) {
     // pivot lane k: the reflector of column k
-    double ss = 0.0;
-#pragma unroll
-    for (int r = k; r < 2 * CS_NY; ++r) ss = fma(Q[r], Q[r], ss);
-    const double x0 = Q[k];
-    const double gk = (x0 >= 0.0) ? -sqrt(ss) : sqrt(ss);
-    const double v0k = x0 - gk;
-    const double vsk = ss - x0 * x0 + v0k * v0k;
+    double gk, v0k, tk;
+    // (the other lanes take 1: a zero column would send the warp through the
+    // out-of-range branches)
+    const double ss = cs_column_ss<L0>(k, Q);
+    const bool on = cs_reflector(c == k ? ss : 1.0, c == k ? Q[k] : 1.0, &gk, &v0k, &tk);
     const double v0 = __shfl_sync(gm, v0k, k, CS_TL);
-    const double vs = __shfl_sync(gm, vsk, k, CS_TL);
+    const double t = __shfl_sync(gm, tk, k, CS_TL);
+    const bool go = __shfl_sync(gm, (int)on, k, CS_TL) != 0;
     double v[2 * CS_NY];
 #pragma unroll
-    for (int r = k + 1; r < 2 * CS_NY; ++r) v[r] = __shfl_sync(gm, Q[r], k, CS_TL);
-    if (vs >= CS_EPS) {
+    for (int r = k + 1; r < 2 * CS_NY; ++r)
+      if (cs_in_reflector<L0>(k, r)) v[r] = __shfl_sync(gm, Q[r], k, CS_TL);
+    if (go) {
       if (c > k) {
-        const double beta = -2.0 / vs;
-        double w = v0 * Q[k];
+        // (the general form: the lanes hold different columns)
+        double w0 = v0 * Q[k], w1 = 0.0;
+        bool first = true;
 #pragma unroll
-        for (int r = k + 1; r < 2 * CS_NY; ++r) w = fma(v[r], Q[r], w);
-        const double bw = beta * w;
+        for (int r = k + 1; r < 2 * CS_NY; ++r)
+          if (cs_in_reflector<L0>(k, r)) {
+            if (((r - k) & 1) == 0) w0 = fma(v[r], Q[r], w0);
+            else if (first) { w1 = v[r] * Q[r]; first = false; }
+            else w1 = fma(v[r], Q[r], w1);
+          }
+        const double bw = -t * (w0 + w1);
         Q[k] = fma(bw, v0, Q[k]);
 #pragma unroll
-        for (int r = k + 1; r < 2 * CS_NY; ++r) Q[r] = fma(bw, v[r], Q[r]);
+        for (int r = k + 1; r < 2 * CS_NY; ++r)
+          if (cs_in_reflector<L0>(k, r)) Q[r] = fma(bw, v[r], Q[r]);
       } else if (c == k) {
         Q[k] = gk;
 #pragma unroll
@@ -1745,9 +1827,13 @@ extern "C" __global__ void k_tree_level(CsBatch bt, int l) {
         const double* src = srcb + (size_t)off * CS_ROWSZ;
         double* dst = dstb + (size_t)off * CS_ROWSZ;
         if (mi < merges) {  // uniform within the lane group
-          cs_merge_lanes(src + (size_t)(2 * mi) * CS_ROWSZ, src + (size_t)(2 * mi + 1) * CS_ROWSZ,
-                         dst + (size_t)mi * CS_ROWSZ, bt.tree + (size_t)(off + ((2 * mi + 1) << l)) * CS_TREESZ,
-                         active);
+          if (l == 0)
+            cs_merge_lanes<true>(src + (size_t)(2 * mi) * CS_ROWSZ, src + (size_t)(2 * mi + 1) * CS_ROWSZ,
+                                 dst + (size_t)mi * CS_ROWSZ, bt.tree + (size_t)(off + 2 * mi + 1) * CS_TREESZ, active);
+          else
+            cs_merge_lanes<false>(src + (size_t)(2 * mi) * CS_ROWSZ, src + (size_t)(2 * mi + 1) * CS_ROWSZ,
+                                  dst + (size_t)mi * CS_ROWSZ, bt.tree + (size_t)(off + ((2 * mi + 1) << l)) * CS_TREESZ,
+                                  active);
         } else if (active) {
           const double* sr = src + (size_t)(nl - 1) * CS_ROWSZ;
           double* dr = dst + (size_t)merges * CS_ROWSZ;
@@ -1767,8 +1853,12 @@ extern "C" __global__ void k_tree_level(CsBatch bt, int l) {
       const double* src = srcb + (size_t)off * CS_ROWSZ;
       double* dst = dstb + (size_t)off * CS_ROWSZ;
       if (mi < merges) {
-        cs_merge_thread(src + (size_t)(2 * mi) * CS_ROWSZ, src + (size_t)(2 * mi + 1) * CS_ROWSZ,
-                        dst + (size_t)mi * CS_ROWSZ, bt.tree + (size_t)(off + ((2 * mi + 1) << l)) * CS_TREESZ);
+        if (l == 0)
+          cs_merge_thread<true>(src + (size_t)(2 * mi) * CS_ROWSZ, src + (size_t)(2 * mi + 1) * CS_ROWSZ,
+                                dst + (size_t)mi * CS_ROWSZ, bt.tree + (size_t)(off + 2 * mi + 1) * CS_TREESZ);
+        else
+          cs_merge_thread<false>(src + (size_t)(2 * mi) * CS_ROWSZ, src + (size_t)(2 * mi + 1) * CS_ROWSZ,
+                                 dst + (size_t)mi * CS_ROWSZ, bt.tree + (size_t)(off + ((2 * mi + 1) << l)) * CS_TREESZ);
       } else {
         const double* sr = src + (size_t)(nl - 1) * CS_ROWSZ;
         double* dr = dst + (size_t)merges * CS_ROWSZ;
@@ -1813,11 +1903,104 @@ extern "C" __global__ void k_tree_level(CsBatch bt, int l) {
 // by Householder QR (the reference: final block QR + np.linalg.solve,
 // solve_babd_system.py:366-423).  Sets the line search going (alpha = 1).
 // top system of instance b, one warp (top: per-warp shared memory)
-__device__ void cs_top_warp(const CsBatch& bt, int b, double* top) {
+// (row: the remaining block row, in global or shared memory)
+#define CS_TOP_LANES (CS_TREE_THREAD && CS_NT <= 16)
+#if CS_TOP_LANES
+// A column per lane in registers, rows unrolled (as cs_merge_lanes); the
+// boundary rows' Jacobian passes through shared memory (top).
+__device__ void cs_top_warp(const CsBatch& bt, int b, const double* row, double* top) {
+  const unsigned full = 0xffffffffu;
+  const int c = threadIdx.x & 31;
+  const int N = bt.N[b], off = bt.off[b];
+  constexpr int W = 2 * CS_NY + CS_NP;
+  if (c == 0) {
+    const double* th = bt.th + (size_t)b * (CS_NTH > 0 ? CS_NTH : 1);
+    double ya[CS_NY], yb[CS_NY], pl[CS_NP > 0 ? CS_NP : 1], r[CS_NY + CS_NP];
+    double Dr[(CS_NY + CS_NP) * W];
+    for (int q = 0; q < CS_NY; ++q) { ya[q] = bt.y[(size_t)off * CS_NY + q]; yb[q] = bt.y[(size_t)(off + N - 1) * CS_NY + q]; }
+    for (int q = 0; q < CS_NP; ++q) pl[q] = bt.p[(size_t)b * CS_NP + q];
+    cs_r(ya, yb, pl, th, r);
+    cs_Dr(ya, yb, pl, th, Dr);
+#pragma unroll
+    for (int q = 0; q < CS_NY + CS_NP; ++q) {
+#pragma unroll
+      for (int e = 0; e < W; ++e) top[q * (W + 1) + e] = Dr[q * W + e];
+      top[q * (W + 1) + W] = cs_neg(r[q]);
+    }
+  }
+  __syncwarp();
+  double q[CS_NT];
+#pragma unroll
+  for (int r = 0; r < CS_NY; ++r) {
+    double v = 0.0;
+    if (c < 2 * CS_NY + CS_NPE) v = row[c * CS_NY + r];
+    else if (c == CS_NT) v = row[(2 * CS_NY + CS_NPE) * CS_NY + r];
+    q[r] = v;
+  }
+#pragma unroll
+  for (int r = 0; r < CS_NY + CS_NP; ++r) q[CS_NY + r] = (c <= CS_NT) ? top[r * (W + 1) + c] : 0.0;
+  double diag = 1.0;
+  cs_static_for<0, CS_NT>([&](auto kc) {
+    constexpr int k = decltype(kc)::value;
+    double s0 = q[k] * q[k], s1 = 0.0;
+    cs_static_for<k + 1, CS_NT>([&](auto rc) {
+      constexpr int r = decltype(rc)::value;
+      if ((r - k) & 1) s1 = fma(q[r], q[r], s1); else s0 = fma(q[r], q[r], s0);
+    });
+    double gk, v0k, tk;
+    const bool on = cs_reflector(c == k ? s0 + s1 : 1.0, c == k ? q[k] : 1.0, &gk, &v0k, &tk);
+    const double v0 = __shfl_sync(full, v0k, k), t = __shfl_sync(full, tk, k);
+    const bool go = __shfl_sync(full, (int)on, k) != 0;
+    if (go) {
+      double w0 = v0 * q[k], w1 = 0.0;
+      double v[CS_NT];
+      cs_static_for<k + 1, CS_NT>([&](auto rc) {
+        constexpr int r = decltype(rc)::value;
+        v[r] = __shfl_sync(full, q[r], k);
+        if ((r - k) & 1) w1 = fma(v[r], q[r], w1); else w0 = fma(v[r], q[r], w0);
+      });
+      const double bw = (c > k) ? -t * (w0 + w1) : 0.0;
+      q[k] = fma(bw, v0, q[k]);
+      cs_static_for<k + 1, CS_NT>([&](auto rc) {
+        constexpr int r = decltype(rc)::value;
+        q[r] = fma(bw, v[r], q[r]);
+      });
+    }
+    if (c == k) diag = go ? gk : q[k];
+  });
+  // back substitution: the right-hand side is lane NT's column
+  const bool zero = c < CS_NT && cs_abskey(diag) == 0ull;
+  const bool sing = __any_sync(full, zero);
+  const double inv = zero ? 0.0 : cs_rcp(diag);
+  cs_static_for<0, CS_NT>([&](auto ic) {
+    constexpr int r = CS_NT - 1 - decltype(ic)::value;
+    const double xr = q[r] * __shfl_sync(full, inv, r);  // (lane NT's)
+    cs_static_for<0, r>([&](auto ec) {
+      constexpr int e = decltype(ec)::value;
+      const double u = __shfl_sync(full, q[e], r);
+      q[e] = (c == CS_NT) ? fma(-u, xr, q[e]) : q[e];
+    });
+    q[r] = (c == CS_NT) ? (sing ? 0.0 : xr) : q[r];
+  });
+  if (c == CS_NT) {
+#pragma unroll
+    for (int e = 0; e < CS_NY; ++e) {
+      bt.dy[(size_t)off * CS_NY + e] = q[e];
+      bt.dy[(size_t)(off + N - 1) * CS_NY + e] = q[CS_NY + e];
+    }
+#pragma unroll
+    for (int e = 0; e < CS_NP; ++e) bt.dp[(size_t)b * CS_NP + e] = q[2 * CS_NY + e];
+    if (sing) bt.inst[b].singular += 1;
+    bt.inst[b].status = ST_LS;
+    bt.inst[b].alpha_ls = 1.0;
+    bt.inst[b].ls_it = 0;
+  }
+  __syncwarp();
+}
+#else
+__device__ void cs_top_warp(const CsBatch& bt, int b, const double* row, double* top) {
   const int lane = threadIdx.x & 31;
   const int N = bt.N[b], off = bt.off[b];
-  const int L = cs_levels(N - 1);
-  const double* row = ((L & 1) ? bt.rows1 : bt.rows0) + (size_t)off * CS_ROWSZ;
   for (int c = lane; c < CS_NT + 1; c += 32) {
     double* col = top + (size_t)c * CS_TLD;
     for (int r = 0; r < CS_NY; ++r) {
@@ -1899,13 +2082,19 @@ __device__ void cs_top_warp(const CsBatch& bt, int b, double* top) {
   }
   __syncwarp();
 }
+#endif  // CS_TOP_LANES
+
+// the block row left of instance b after its last tree level
+__device__ __forceinline__ const double* cs_top_row(const CsBatch& bt, int b) {
+  return ((cs_levels(bt.N[b] - 1) & 1) ? bt.rows1 : bt.rows0) + (size_t)bt.off[b] * CS_ROWSZ;
+}
 
 extern "C" __global__ void k_top(CsBatch bt) {
   extern __shared__ double smem[];
   const int wpc = blockDim.x >> 5, w = threadIdx.x >> 5;
   double* top = smem + (size_t)w * CS_TLD * (CS_NT + 1);
   const int njac = bt.nlist[1];
-  for (int k = blockIdx.x * wpc + w; k < njac; k += gridDim.x * wpc) cs_top_warp(bt, bt.jac[k], top);
+  for (int k = blockIdx.x * wpc + w; k < njac; k += gridDim.x * wpc) cs_top_warp(bt, bt.jac[k], cs_top_row(bt, bt.jac[k]), top);
 }
 #endif  // !CS_BIG_TREE
 
@@ -1956,51 +2145,64 @@ extern "C" __global__ void k_backsub_level(CsBatch bt, int l) {
 }
 
 #if !CS_BIG_TREE && CS_TREE_THREAD && CS_QC <= 32
-// The upper tree levels l >= l_lo of every instance on the jac list, its top
-// system and the back substitution of those levels, one CTA per instance:
-// levels with at most a few merges each, which as launches of their own cost
-// a launch and a work-list lookup apiece for a few dependent merges.  Merges
-// by groups of CS_TL lanes (cs_merge_lanes), back substitution by thread
-// (cs_backsub_thread): the per-level kernels' arithmetic, so the same bits.
-// Levels below l_lo go through k_tree_level / k_backsub_level before and
-// after this launch.
-extern "C" __global__ void __launch_bounds__(128) k_upper(CsBatch bt, int l_lo) {
-  extern __shared__ double smem[];
+// The upper tree levels l >= l_first of every instance on the jac list (at most
+// CS_UROWS block rows there), its top system and the back substitution of those
+// levels, one CTA per instance: as launches of their own these levels cost a
+// launch and a work-list lookup apiece for a few dependent merges.  Merges by
+// groups of CS_TL lanes (cs_merge_lanes), back substitution by thread
+// (cs_backsub_thread): the per-level kernels' arithmetic, so the same bits.  Rows
+// and tree records stay in shared memory: nothing outside this launch reads
+// them, and each level is otherwise a round trip to L2.  Levels below go
+// through k_tree_level / k_backsub_level before and after this launch.
+// Measured (4 levels and the top system of 333 instances): 84 -> 64 us.
+#define CS_UROWS 16
+extern "C" __global__ void __launch_bounds__(128) k_upper(CsBatch bt, int l_first) {
+  __shared__ double rows[2][CS_UROWS * CS_ROWSZ];
+  __shared__ double recs[CS_UROWS * CS_TREESZ];  // of the node at position e (units of 2^l_lo)
+  __shared__ double top[(CS_NY + CS_NP) * (2 * CS_NY + CS_NP + 1)];
+  __shared__ double nodes[(CS_UROWS + 1) * CS_NY];
   const int groups = blockDim.x / CS_TL, grp = threadIdx.x / CS_TL, c = threadIdx.x & (CS_TL - 1);
   const int njac = bt.nlist[1];
   for (int k = blockIdx.x; k < njac; k += gridDim.x) {
     const int b = bt.jac[k];
     const int off = bt.off[b];
     const int n0 = bt.N[b] - 1;
-    const int L = cs_levels(n0);
-    for (int l = l_lo; l < L; ++l) {
+    const int L = cs_levels(n0), l_lo = min(l_first, L);  // (a short mesh may be done below l_first)
+    const int nr = cs_rows_at(n0, l_lo);
+    const double* src = ((l_lo & 1) ? bt.rows1 : bt.rows0) + (size_t)off * CS_ROWSZ;
+    for (int e = threadIdx.x; e < nr * CS_ROWSZ; e += blockDim.x) rows[0][e] = src[e];
+    __syncthreads();
+    int cur = 0;
+    for (int l = l_lo; l < L; ++l, cur ^= 1) {
       const int nl = cs_rows_at(n0, l);
       const int merges = nl >> 1, items = (nl + 1) >> 1;
-      const double* src = ((l & 1) ? bt.rows1 : bt.rows0) + (size_t)off * CS_ROWSZ;
-      double* dst = ((l & 1) ? bt.rows0 : bt.rows1) + (size_t)off * CS_ROWSZ;
+      const double* in = rows[cur];
+      double* out = rows[cur ^ 1];
       for (int mi = grp; mi < items; mi += groups) {  // uniform within a lane group
         if (mi < merges) {
-          cs_merge_lanes(src + (size_t)(2 * mi) * CS_ROWSZ, src + (size_t)(2 * mi + 1) * CS_ROWSZ,
-                         dst + (size_t)mi * CS_ROWSZ, bt.tree + (size_t)(off + ((2 * mi + 1) << l)) * CS_TREESZ, true);
+          cs_merge_lanes<false>(in + 2 * mi * CS_ROWSZ, in + (2 * mi + 1) * CS_ROWSZ, out + mi * CS_ROWSZ,
+                                recs + ((2 * mi + 1) << (l - l_lo)) * CS_TREESZ, true);
         } else {
-          const double* sr = src + (size_t)(nl - 1) * CS_ROWSZ;
-          double* dr = dst + (size_t)merges * CS_ROWSZ;
-          for (int q = c; q < CS_ROWSZ; q += CS_TL) dr[q] = sr[q];
+          for (int q = c; q < CS_ROWSZ; q += CS_TL) out[merges * CS_ROWSZ + q] = in[(nl - 1) * CS_ROWSZ + q];
         }
       }
       __syncthreads();
     }
-    if (threadIdx.x < 32) cs_top_warp(bt, b, smem);
+    if (threadIdx.x < 32) cs_top_warp(bt, b, rows[cur], top);
+    __syncthreads();
+    for (int e = threadIdx.x; e < 2 * CS_NY; e += blockDim.x) {
+      const int a = e < CS_NY ? e : e - CS_NY;
+      nodes[(e < CS_NY ? 0 : nr) * CS_NY + a] = bt.dy[(size_t)(off + (e < CS_NY ? 0 : n0)) * CS_NY + a];
+    }
     __syncthreads();
     const double* dpv = bt.dp + (size_t)b * CS_NP;
     for (int l = L - 1; l >= l_lo; --l) {
-      const int merges = cs_rows_at(n0, l) >> 1;
+      const int merges = cs_rows_at(n0, l) >> 1, sh = l - l_lo;
       for (int mi = threadIdx.x; mi < merges; mi += blockDim.x) {
-        const int mid = (2 * mi + 1) << l, left = (2 * mi) << l;
-        int right = (2 * mi + 2) << l;
-        if (right > n0) right = n0;
-        cs_backsub_thread(bt.tree + (size_t)(off + mid) * CS_TREESZ, bt.dy + (size_t)(off + left) * CS_NY,
-                          bt.dy + (size_t)(off + right) * CS_NY, dpv, bt.dy + (size_t)(off + mid) * CS_NY);
+        const int mid = (2 * mi + 1) << sh, left = (2 * mi) << sh, right = min((2 * mi + 2) << sh, nr);
+        double* ym = nodes + mid * CS_NY;
+        cs_backsub_thread(recs + mid * CS_TREESZ, nodes + left * CS_NY, nodes + right * CS_NY, dpv, ym);
+        for (int q = 0; q < CS_NY; ++q) bt.dy[(size_t)(off + (mid << l_lo)) * CS_NY + q] = ym[q];
       }
       __syncthreads();
     }
@@ -2135,8 +2337,8 @@ extern "C" __global__ void __launch_bounds__(256) k_babd_cta(CsBatch bt) {
 #if CS_TREE_THREAD
       for (int mi = threadIdx.x; mi < items; mi += blockDim.x) {
         if (mi < merges) {
-          cs_merge_thread(src + (size_t)(2 * mi) * CS_ROWSZ, src + (size_t)(2 * mi + 1) * CS_ROWSZ,
-                          dst + (size_t)mi * CS_ROWSZ, bt.tree + (size_t)(off + ((2 * mi + 1) << l)) * CS_TREESZ);
+          cs_merge_thread<false>(src + (size_t)(2 * mi) * CS_ROWSZ, src + (size_t)(2 * mi + 1) * CS_ROWSZ,
+                                 dst + (size_t)mi * CS_ROWSZ, bt.tree + (size_t)(off + ((2 * mi + 1) << l)) * CS_TREESZ);
         } else {
           const double* sr = src + (size_t)(nl - 1) * CS_ROWSZ;
           double* dr = dst + (size_t)merges * CS_ROWSZ;
@@ -2159,7 +2361,7 @@ extern "C" __global__ void __launch_bounds__(256) k_babd_cta(CsBatch bt) {
       __syncthreads();
     }
     // ---- top system (warp 0)
-    if (w == 0) cs_top_warp(bt, b, top);
+    if (w == 0) cs_top_warp(bt, b, cs_top_row(bt, b), top);
     __syncthreads();
     // ---- back substitution down
     const double* dpv = bt.dp + (size_t)b * CS_NP;

@@ -324,7 +324,7 @@ struct cs_module {
   size_t babd_cta_smem;
   // k_upper (upper tree levels, top and their back substitution, CTA per
   // instance): 0 when the block rows are too large for lane merges
-  size_t upper_smem = 0;
+  bool upper = false;
   int upper_grid = 0;
   // one wave of resident CTAs: grids of the grid-stride kernels k_residual and
   // k_tree_level (small block rows), so that launches with little work do not
@@ -573,7 +573,7 @@ extern "C" int cs_module_load(const cs_module_desc* d, cs_module** out) {
     M->babd_cta_smem = top_per + (size_t)8 * qld * qc * sizeof(double);
     M->top_smem = top_per * M->top_wpc;
     // CS_TREE_THREAD && CS_QC <= 32 in cs_kernels.cuh (lane merges)
-    if (2 * M->ny * qc <= 128 && qc <= 32 && top_per <= (size_t)smem_optin) M->upper_smem = top_per;
+    if (2 * M->ny * qc <= 128 && qc <= 32) M->upper = true;
   }
 
   std::string src = build_source(d, M->big_cond, M->big_tree, M->prec, M->big_tree ? M->prec_tree : 0, smem_optin);
@@ -696,11 +696,9 @@ extern "C" int cs_module_load(const cs_module_desc* d, cs_module** out) {
       M->tree_small_grid = M->sms * std::max(1, std::min(pt, 8));
     }
   }
-  if (M->upper_smem) {
-    if (M->upper_smem > 48 * 1024)
-      CS_CU(g_drv.funcSetAttribute(M->f_upper, CU_FUNC_ATTRIBUTE_MAX_DYNAMIC_SHARED_SIZE_BYTES, (int)M->upper_smem));
+  if (M->upper) {
     int pu = 0;
-    CS_CU(g_drv.occupancy(&pu, M->f_upper, 128, M->upper_smem));
+    CS_CU(g_drv.occupancy(&pu, M->f_upper, 128, 0));
     M->upper_grid = M->sms * std::max(1, std::min(pu, 16));
   }
   if (M->babd_cta_smem > (size_t)smem_optin) M->babd_cta_smem = 0;  // per-level kernels only
@@ -1054,7 +1052,7 @@ static bool use_cta_path(const cs_batch* bt) {
 // or babd_path 2 asks for one launch per level).
 static const int kUpperLevels = 4;
 static int upper_levels(const cs_batch* bt, int nlvl) {
-  if (!bt->M->upper_smem || bt->opts.babd_path == 2) return nlvl;
+  if (!bt->M->upper || bt->opts.babd_path == 2) return nlvl;
   return std::max(0, nlvl - kUpperLevels);
 }
 
@@ -1090,10 +1088,10 @@ static int run_direction(cs_batch* bt, CsBatchDev& v, int nlvl) {
     if (M->big_tree) CS_TRY(launch_k(bt, M->f_tree_level, gtree, 256, M->tree_smem, a, 1));
     else CS_TRY(launch_k(bt, M->f_tree_level, gtree, 128, M->tree_smem, a, 1));
   }
-  if (M->upper_smem && bt->opts.babd_path != 2) {
+  if (M->upper && bt->opts.babd_path != 2) {
     int lo = l_lo;
     void* a[] = {&v, &lo};
-    CS_TRY(launch_k(bt, M->f_upper, capped_inst(bt, (unsigned)std::min(M->upper_grid, bt->B)), 128, M->upper_smem, a, 1));
+    CS_TRY(launch_k(bt, M->f_upper, capped_inst(bt, (unsigned)std::min(M->upper_grid, bt->B)), 128, 0, a, 1));
   } else {
     void* a[] = {&v};
     if (M->big_tree)
