@@ -35,7 +35,7 @@
 //                                                      solve_babd_system.py:161-572, collocation_solver_parallel_2d_shared.py:1619-1650
 //   k_lists          (none: compacts the work of the batch every super-step)
 //   k_decide/k_accept  Newton loop and line search    collocation_solver_parallel_2d_shared.py:105-180
-//   k_segres         compute_segment_residual_kernel(2) collocation_solver_parallel_2d_shared.py:1833-2013
+//   k_segres(_list)  compute_segment_residual_kernel(2) collocation_solver_parallel_2d_shared.py:1833-2013
 //   k_remesh_*       recover_solution_kernel + remesh  collocation_solver_parallel_2d_shared.py:2049-2311
 
 #define CS_S (CS_M * (CS_NY + CS_NZ))          // stage unknowns per interval
@@ -85,6 +85,7 @@ struct CsConsts {
   double tol, alpha_m, beta;
   int max_iter, max_mesh, max_nodes, min_nodes, max_ls;
   int ls_grow;  // trials of a new line search after one that rejected some (cs_opts.ls_grow)
+  int rtype, scale, res2;  // segment residual estimate
 };
 
 struct CsBatch {
@@ -122,12 +123,14 @@ struct CsBatch {
   long long* jac_pre;       // [B+1] prefix of interval counts
   long long* acc_pre;       // [B+1] prefix of node counts
   long long* lvl_pre;       // [CS_MAXLVL][B+1] prefix of tree items per level over jac
-  int* nlist;               // [4] nact, njac, nacc, -
+  int* nlist;               // [4] nact, njac, nacc, nseg
   unsigned long long* trials;  // [B][CS_LSW] residual norms of line-search trials 1.. (bits)
   // large stage systems (CS_BIG): a slab of global memory per CTA
   double* wsp;              // [wsp_ctas][wsp_stride]
   long long wsp_stride;     // doubles per CTA
   int wsp_ctas, wsp_pad;
+  int* seg;                 // [B] instances whose segment residual is due
+  long long* seg_pre;       // [B+1] prefix of node counts
   unsigned char* zform;     // [T] register condensation: 1 if the z rows of X hold g_z^-1 [g_y g_p g] (0: the solution)
 };
 
@@ -442,9 +445,7 @@ __device__ void cs_iteration_start(CsInst& s, int N, const CsConsts& c, bool cou
   s.jac_count += 1;
 }
 
-extern "C" __global__ void k_decide(CsBatch bt, CsConsts c) {
-  int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= bt.B) return;
+__device__ __forceinline__ void cs_decide(const CsBatch& bt, const CsConsts& c, int b) {
   CsInst s = bt.inst[b];
   s.accepted = 0;
   s.need_jac = 0;
@@ -512,6 +513,11 @@ extern "C" __global__ void k_decide(CsBatch bt, CsConsts c) {
   bt.inst[b] = s;
 }
 
+extern "C" __global__ void k_decide(CsBatch bt, CsConsts c) {
+  const int b = blockIdx.x * blockDim.x + threadIdx.x;
+  if (b < bt.B) cs_decide(bt, c, b);
+}
+
 // x += alpha_ls * dx for instances whose trial was accepted (items: their nodes)
 extern "C" __global__ void k_accept(CsBatch bt) {
   const int nacc = bt.nlist[2];
@@ -539,11 +545,15 @@ extern "C" __global__ void k_accept(CsBatch bt) {
 }
 
 // ------------------------------------------------------------------------
-// Work lists.  One CTA of 1024 threads scans the instances:
-//   mode 0: act = instances in FRESH or LS; jac, acc empty
+// Work lists.  One CTA (a thread per instance, at most 1024) scans the
+// instances:
+//   mode 0: act = instances in FRESH or LS; the others empty
 //   mode 1: (after k_decide) act = FRESH/LS or needing a Jacobian, jac =
-//           needing a Jacobian, acc = accepted trials; plus, for each tree
-//           level l < nlvl, the prefix of that level's items over jac.
+//           needing a Jacobian, acc = accepted trials, seg = converged; plus,
+//           for each tree level l < nlvl, the prefix of that level's items
+//           over jac.
+//   mode 2: mode 1 with k_decide's work done first (batches small enough for
+//           one CTA to walk: a launch less per super-step)
 __device__ long long cs_block_scan(long long v, long long* sh, long long* total) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
   long long x = v;
@@ -597,12 +607,16 @@ __device__ __forceinline__ long long cs_res_items(const CsInst& s, int N) {
   return (long long)(N - 1) * t;
 }
 
-extern "C" __global__ void k_lists(CsBatch bt, int mode, int nlvl) {
+extern "C" __global__ void __launch_bounds__(1024) k_lists(CsBatch bt, CsConsts c, int mode, int nlvl) {
   __shared__ long long sh[32];
   const int B = bt.B;
+  if (mode == 2) {
+    for (int b = threadIdx.x; b < B; b += blockDim.x) cs_decide(bt, c, b);
+    __syncthreads();
+  }
   const CsInst* I = bt.inst;
   const int* N = bt.N;
-  int nact, njac = 0, nacc = 0;
+  int nact, njac = 0, nacc = 0, nseg = 0;
   if (mode == 0) {
     nact = cs_build_list(B, [&](int b) { int st = I[b].status; return st == ST_FRESH || st == ST_LS; },
                          [&](int b) { return cs_res_items(I[b], N[b]); }, bt.act, bt.act_pre, sh);
@@ -614,6 +628,8 @@ extern "C" __global__ void k_lists(CsBatch bt, int mode, int nlvl) {
                          bt.jac, bt.jac_pre, sh);
     nacc = cs_build_list(B, [&](int b) { return I[b].accepted != 0; }, [&](int b) { return (long long)N[b]; },
                          bt.acc, bt.acc_pre, sh);
+    nseg = cs_build_list(B, [&](int b) { return I[b].status == ST_SEG; }, [&](int b) { return (long long)N[b]; }, bt.seg,
+                         bt.seg_pre, sh);
     const int* J = bt.jac;
     for (int l = 0; l < nlvl && l < CS_MAXLVL; ++l)
       cs_build_list(njac, [&](int k) { return true; }, [&](int k) { return cs_level_items(N[J[k]] - 1, l); },
@@ -623,6 +639,7 @@ extern "C" __global__ void k_lists(CsBatch bt, int mode, int nlvl) {
     bt.nlist[0] = nact;
     bt.nlist[1] = njac;
     bt.nlist[2] = nacc;
+    bt.nlist[3] = nseg;
   }
 }
 
@@ -3902,13 +3919,10 @@ __device__ __forceinline__ void cs_gauss_point(const double* yi, const double* y
   }
 }
 
-extern "C" __global__ void k_segres(CsBatch bt, double tol, int rtype, int scale, int res2) {
-  int slot = blockIdx.x * blockDim.x + threadIdx.x;
-  if (slot >= bt.T) return;
-  int b = bt.inst_of[slot];
-  int i = slot - bt.off[b];
-  int N = bt.N[b];
-  if (bt.inst[b].status != ST_SEG) return;
+// node slot `slot` of instance b
+__device__ __forceinline__ void cs_segres_node(const CsBatch& bt, int slot, int b, double tol, int rtype, int scale, int res2) {
+  const int i = slot - bt.off[b];
+  const int N = bt.N[b];
   const double* th = bt.th + (size_t)b * (CS_NTH > 0 ? CS_NTH : 1);
   double pl[CS_NP > 0 ? CS_NP : 1];
   for (int k = 0; k < CS_NP; ++k) pl[k] = bt.p[(size_t)b * CS_NP + k];
@@ -3984,27 +3998,76 @@ extern "C" __global__ void k_segres(CsBatch bt, double tol, int rtype, int scale
   atomicMax(&bt.inst[b].res_bits, bits);
 }
 
-// after k_segres: accept the mesh, continue the continuation, or ask for a remesh
-extern "C" __global__ void k_mesh_decide(CsBatch bt, CsConsts c) {
-  int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= bt.B) return;
-  CsInst s = bt.inst[b];
-  if (s.status != ST_SEG) return;
-  s.max_res = cs_from_bits(s.res_bits);
-  s.res_bits = 0ull;
-  s.seg_count += 1;
-  if (s.max_res > 1.0) {
-    s.status = ST_REMESH;
-  } else if (s.alpha <= c.alpha_m) {
-    s.status = ST_DONE;
-  } else {
-    s.alpha *= c.beta;
-    s.alphacal += 1;
-    s.status = ST_FRESH;
-    s.it = 0;
+// every slot of the instances in SEG (stage entry point)
+extern "C" __global__ void k_segres(CsBatch bt, double tol, int rtype, int scale, int res2) {
+  const int slot = blockIdx.x * blockDim.x + threadIdx.x;
+  if (slot >= bt.T) return;
+  const int b = bt.inst_of[slot];
+  if (bt.inst[b].status == ST_SEG) cs_segres_node(bt, slot, b, tol, rtype, scale, res2);
+}
+
+// The mesh phase inside the super-step: the nodes of the instances that have
+// just converged (seg list), then, in one CTA, their decision -- accept the
+// mesh, go on with the next continuation parameter, or ask for a remesh.  An
+// instance that goes on joins the residual list at once.  Before, the host did
+// this between Newton phases: for a continuation of a hundred steps on a small
+// mesh, a hundred times a synchronisation, a record round trip, and the empty
+// super-steps launched until the next check.
+extern "C" __global__ void k_segres_list(CsBatch bt, CsConsts c) {
+  const int n = bt.nlist[3];
+  if (n == 0) return;
+  const long long total = bt.seg_pre[n];
+  for (long long w = (long long)blockIdx.x * blockDim.x + threadIdx.x; w < total; w += (long long)gridDim.x * blockDim.x) {
+    const int k = cs_find(bt.seg_pre, n, w);
+    const int b = bt.seg[k];
+    cs_segres_node(bt, bt.off[b] + (int)(w - bt.seg_pre[k]), b, c.tol, c.rtype, c.scale, c.res2);
   }
-  bt.inst[b].max_res = s.max_res;
-  bt.inst[b] = s;
+}
+
+extern "C" __global__ void __launch_bounds__(1024) k_mesh_decide(CsBatch bt, CsConsts c) {
+  __shared__ long long sh[32];
+  const int n = bt.nlist[3];
+  if (n == 0) return;
+  int nact = bt.nlist[0];
+  long long items = bt.act_pre[nact];
+  __syncthreads();
+  for (int base = 0; base < n; base += blockDim.x) {
+    const int k = base + threadIdx.x;
+    int b = -1, fresh = 0;
+    if (k < n) {
+      b = bt.seg[k];
+      CsInst s = bt.inst[b];
+      s.max_res = cs_from_bits(s.res_bits);
+      s.res_bits = 0ull;
+      s.seg_count += 1;
+      if (s.max_res > 1.0) {
+        s.status = ST_REMESH;
+      } else if (s.alpha <= c.alpha_m) {
+        s.status = ST_DONE;
+      } else {
+        s.alpha *= c.beta;
+        s.alphacal += 1;
+        s.status = ST_FRESH;
+        s.it = 0;
+        fresh = 1;
+      }
+      bt.inst[b] = s;
+    }
+    long long tf, tw;
+    const long long wv = fresh ? (long long)(bt.N[b] - 1) : 0ll;
+    const long long pf = cs_block_scan((long long)fresh, sh, &tf);
+    const long long pw = cs_block_scan(wv, sh, &tw);
+    if (fresh) {
+      bt.act[nact + pf] = b;
+      bt.act_pre[nact + pf] = items + pw;
+    }
+    nact += (int)tf;
+    items += tw;
+  }
+  if (threadIdx.x == 0) {
+    bt.act_pre[nact] = items;
+    bt.nlist[0] = nact;
+  }
 }
 
 // ------------------------------------------------------------------------

@@ -4,12 +4,12 @@
 //
 // The driver follows collocation_solver_parallel (collocation_solver_parallel_2d_shared.py:36-251)
 // but keeps the whole Newton loop on the device: each "super-step" launches
-//   k_residual -> k_decide -> k_accept -> k_condense -> k_babd
+//   k_residual -> k_decide -> k_accept -> k_condense -> k_babd -> k_segres
 // and every instance advances its own state machine (fresh residual, line
-// search trial, converged, failed) inside those kernels.  The host only
-// checks, every few super-steps, whether any instance is still in Newton, and
-// runs the mesh phase (segment residual, remesh with repacking) between
-// Newton phases.
+// search trial, converged, next continuation parameter, done, failed) inside
+// those kernels.  The host only checks, every few super-steps, whether any
+// instance is still in Newton, and remeshes (with repacking) between Newton
+// phases.
 #include <cuda.h>
 #include <cuda_profiler_api.h>
 #include <cuda_runtime.h>
@@ -102,6 +102,7 @@ struct CsConsts {
   double tol, alpha_m, beta;
   int max_iter, max_mesh, max_nodes, min_nodes, max_ls;
   int ls_grow;
+  int rtype, scale, res2;
 };
 
 // Must match struct CsBatch in cs_kernels.cuh.
@@ -142,6 +143,8 @@ struct CsBatchDev {
   double* wsp;
   long long wsp_stride;
   int wsp_ctas, wsp_pad;
+  int* seg;
+  long long* seg_pre;
   unsigned char* zform;
 };
 
@@ -315,7 +318,7 @@ struct cs_module {
   int ny, nz, np, npe, nth, m, s, nrhs, cgw;
   size_t rowsz, treesz;
   CUmodule mod = nullptr;
-  CUfunction f_form_initial, f_residual, f_decide, f_accept, f_condense, f_segres, f_mesh_decide,
+  CUfunction f_form_initial, f_residual, f_decide, f_accept, f_condense, f_segres, f_segres_list, f_mesh_decide,
       f_remesh_count, f_remesh_write, f_repack, f_znodes, f_lists, f_tree_level, f_top, f_backsub_level, f_recover,
       f_babd_cta, f_upper;
   // FP64 refinement of the direction when the tree merges run on the tensor
@@ -598,7 +601,8 @@ extern "C" int cs_module_load(const cs_module_desc* d, cs_module** out) {
     const char* name;
   } fns[] = {{&M->f_form_initial, "k_form_initial"}, {&M->f_residual, "k_residual"},   {&M->f_decide, "k_decide"},
              {&M->f_accept, "k_accept"},             {&M->f_condense, "k_condense"},
-             {&M->f_segres, "k_segres"},             {&M->f_mesh_decide, "k_mesh_decide"},
+             {&M->f_segres, "k_segres"},             {&M->f_segres_list, "k_segres_list"},
+             {&M->f_mesh_decide, "k_mesh_decide"},
              {&M->f_remesh_count, "k_remesh_count"}, {&M->f_remesh_write, "k_remesh_write"},
              {&M->f_repack, "k_repack"},             {&M->f_znodes, "k_znodes"},
              {&M->f_lists, "k_lists"},               {&M->f_tree_level, "k_tree_level"},
@@ -776,7 +780,7 @@ struct cs_batch {
   std::vector<int> hN, hoff;
   cs_opts opts;
   // work lists
-  DBuf l_act, l_jac, l_acc, l_actp, l_jacp, l_accp, l_lvlp, l_n;
+  DBuf l_act, l_jac, l_acc, l_seg, l_actp, l_jacp, l_accp, l_segp, l_lvlp, l_n;
   int* h_n = nullptr;  // pinned copy of nlist (8 ints: the lists' counts, then k_spares' counts)
   cs_progress_fn progress = nullptr;
   void* progress_user = nullptr;
@@ -926,6 +930,8 @@ static CsBatchDev devview(cs_batch* bt) {
   v.acc_pre = (long long*)bt->l_accp.p;
   v.lvl_pre = (long long*)bt->l_lvlp.p;
   v.nlist = (int*)bt->l_n.p;
+  v.seg = (int*)bt->l_seg.p;
+  v.seg_pre = (long long*)bt->l_segp.p;
   v.trials = (unsigned long long*)bt->dtrials.p;
   if (bt->M->big) {
     v.wsp = (double*)bt->wsp.p;
@@ -1056,10 +1062,18 @@ static int upper_levels(const cs_batch* bt, int nlvl) {
   return std::max(0, nlvl - kUpperLevels);
 }
 
-static int run_lists(cs_batch* bt, CsBatchDev& v, int mode, int nlvl) {
-  void* args[] = {&v, &mode, &nlvl};
-  return launch(bt, bt->M->f_lists, 1, 1024, 0, args);
+// a thread per instance up to 1024: a small batch's scans stay in few warps
+static int run_lists(cs_batch* bt, CsBatchDev& v, int mode, int nlvl, const CsConsts* c = nullptr) {
+  CsConsts cc;
+  memset(&cc, 0, sizeof(cc));
+  if (c) cc = *c;
+  void* args[] = {&v, &cc, &mode, &nlvl};
+  return launch(bt, bt->M->f_lists, 1, (unsigned)std::min(1024, (bt->B + 31) / 32 * 32), 0, args);
 }
+
+// up to this many instances one CTA takes the Newton decisions along with the
+// work lists
+static const int kDecideInLists = 4096;
 
 // Newton direction for the instances on the jac list: tree levels up, top
 // system, back substitution down, stage recovery.
@@ -1149,6 +1163,9 @@ static CsConsts consts_of(const cs_opts& o) {
   c.min_nodes = o.min_nodes;
   c.max_ls = o.max_linesearch;
   c.ls_grow = o.ls_grow;
+  c.rtype = o.residual_type;
+  c.scale = o.scale_by_time;
+  c.res2 = o.residual2;
   return c;
 }
 
@@ -1186,6 +1203,7 @@ extern "C" int cs_batch_create(cs_module* M, int batch, long long node_capacity,
       (rc = dalloc(bt->dcounters, 64)) || (rc = dalloc(bt->l_act, batch * sizeof(int))) ||
       (rc = dalloc(bt->dtrials, (size_t)batch * CS_LSW * sizeof(unsigned long long))) ||
       (rc = dalloc(bt->l_jac, batch * sizeof(int))) || (rc = dalloc(bt->l_acc, batch * sizeof(int))) ||
+      (rc = dalloc(bt->l_seg, batch * sizeof(int))) || (rc = dalloc(bt->l_segp, (batch + 1) * sizeof(long long))) ||
       (rc = dalloc(bt->l_actp, (batch + 1) * sizeof(long long))) ||
       (rc = dalloc(bt->l_jacp, (batch + 1) * sizeof(long long))) ||
       (rc = dalloc(bt->l_accp, (batch + 1) * sizeof(long long))) ||
@@ -1212,7 +1230,7 @@ extern "C" void cs_batch_free(cs_batch* bt) {
   DBuf* all[] = {&bt->dN, &bt->doff, &bt->doff2, &bt->dp, &bt->dth, &bt->ddp, &bt->dinst, &bt->dcounters, &bt->dtrials,
                  &bt->inst_of, &bt->dy, &bt->dydot, &bt->dzt, &bt->X, &bt->rows0, &bt->rows1, &bt->tree, &bt->res, &bt->zform,
                  &bt->iN, &bt->ioff, &bt->it, &bt->iy, &bt->iz, &bt->ip, &bt->l_act, &bt->l_jac, &bt->l_acc,
-                 &bt->l_actp, &bt->l_jacp, &bt->l_accp, &bt->l_lvlp, &bt->l_n, &bt->wsp,
+                 &bt->l_actp, &bt->l_jacp, &bt->l_accp, &bt->l_seg, &bt->l_segp, &bt->l_lvlp, &bt->l_n, &bt->wsp,
                  &bt->rows_keep, &bt->dy_keep, &bt->dp_keep};
   for (DBuf* b : all) dfree(*b);
   cs_text_scratch_free(&bt->text);
@@ -1368,14 +1386,22 @@ static int super_step(cs_batch* bt, const CsConsts& c, int nlvl) {
   bt->super_steps += 1;
   CsConsts cc = c;
   void* dargs[] = {&v, &cc};
-  CS_TRY(run_insts(bt, M->f_decide, dargs));
-  CS_TRY(run_lists(bt, v, 1, use_cta_path(bt) ? 0 : nlvl));
+  const int lists = use_cta_path(bt) ? 0 : upper_levels(bt, nlvl);  // levels with a launch of their own
+  if (bt->B <= kDecideInLists) {
+    CS_TRY(run_lists(bt, v, 2, lists, &c));
+  } else {
+    CS_TRY(run_insts(bt, M->f_decide, dargs));
+    CS_TRY(run_lists(bt, v, 1, lists));
+  }
   {
     void* args[] = {&v};
     CS_TRY(launch(bt, M->f_accept, capped(bt, g, 1, 256), 256, 0, args));
   }
   CS_TRY(run_condense(bt, v));
-  return run_direction(bt, v, nlvl);
+  CS_TRY(run_direction(bt, v, nlvl));
+  // the mesh phase of the instances that converged in this super-step
+  CS_TRY(launch(bt, M->f_segres_list, capped(bt, g, 1, 256), 256, 0, dargs));
+  return launch(bt, M->f_mesh_decide, 1, (unsigned)std::min(1024, (bt->B + 31) / 32 * 32), 0, dargs);
 }
 
 // A CUDA graph of `reps` super-steps for the current layout (re-captured when
@@ -1554,7 +1580,7 @@ extern "C" int cs_solve(cs_batch* bt, const cs_opts* opts) {
         if (use_graph) {
           cudaError_t e = cudaGraphLaunch(bt->graph[cta ? 1 : 0], bt->stream);
           if (e != cudaSuccess) rc = set_err(CS_ERR_CUDA, std::string("graph launch: ") + cudaGetErrorString(e));
-          bt->launches += cta ? 7 : 9 + 2 * upper_levels(bt, nlvl);
+          bt->launches += (cta ? 8 : 8 + 2 * upper_levels(bt, nlvl)) + (bt->B > kDecideInLists ? 1 : 0);
           bt->super_steps += 1;
         } else {
           rc = super_step(bt, c, nlvl);
@@ -1583,15 +1609,8 @@ extern "C" int cs_solve(cs_batch* bt, const cs_opts* opts) {
       }
     }
     if (rc != CS_OK) break;
-    // ---- mesh phase
-    CsBatchDev v = devview(bt);
-    double tol = o.tol;
-    int rtype = o.residual_type, scale = o.scale_by_time, res2 = o.residual2;
-    void* as[] = {&v, &tol, &rtype, &scale, &res2};
-    if ((rc = launch(bt, bt->M->f_segres, cdiv(bt->T, 256), 256, 0, as)) != CS_OK) break;
-    CsConsts cc = c;
-    void* am[] = {&v, &cc};
-    if ((rc = run_insts(bt, bt->M->f_mesh_decide, am)) != CS_OK) break;
+    // ---- remesh: the segment residuals and their decisions were part of the
+    //      super-steps
     if ((rc = read_inst(bt, hi)) != CS_OK) break;
     bool any_remesh = false, any_newton = false;
     for (auto& s : hi) {
@@ -1815,7 +1834,7 @@ extern "C" int cs_stage_newton_direction(cs_batch* bt, double alpha, double* row
   CS_TRY(set_all_status(bt, ST_FRESH, alpha, 1));
   CsBatchDev v = devview(bt);
   const int nlvl = tree_levels(bt);
-  CS_TRY(run_lists(bt, v, 1, use_cta_path(bt) ? 0 : nlvl));
+  CS_TRY(run_lists(bt, v, 1, use_cta_path(bt) ? 0 : upper_levels(bt, nlvl)));
   CS_TRY(run_condense(bt, v));
   const size_t d = sizeof(double);
   cudaStream_t st = bt->stream;
