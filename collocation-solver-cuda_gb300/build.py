@@ -21,14 +21,14 @@ ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 
 
 def _kernels_header():
-    """cs_umma.cuh + cs_kernels.cuh as a C string constant (the NVRTC program
-    text after the problem-specific prelude)."""
+    """cs_umma.cuh, cs_fp64.cuh and cs_kernels.cuh as a C string constant (the
+    NVRTC program text after the problem-specific prelude)."""
     os.makedirs(BUILD, exist_ok=True)
-    src = open(os.path.join(CSRC, "cs_umma.cuh")).read() + "\n" + open(os.path.join(CSRC, "cs_kernels.cuh")).read()
+    src = "\n".join(open(os.path.join(CSRC, f)).read() for f in ("cs_umma.cuh", "cs_fp64.cuh", "cs_kernels.cuh"))
     out = os.path.join(BUILD, "cs_kernels_src.h")
     delim = "CSKSRC"
     assert (")" + delim + '"') not in src
-    text = "// generated from cs_umma.cuh and cs_kernels.cuh by build.py\n"
+    text = "// generated from cs_umma.cuh, cs_fp64.cuh and cs_kernels.cuh by build.py\n"
     # split into chunks: some compilers limit the length of one string literal
     chunks = [src[i:i + 16000] for i in range(0, len(src), 16000)]
     text += "static const char cs_kernels_source[] =\n"
@@ -52,7 +52,7 @@ def build_library(force=False, verbose=False):
     hdr = _kernels_header()
     sources = [os.path.join(CSRC, "cs_runtime.cu"), os.path.join(CSRC, "cs_babd.cu"), os.path.join(CSRC, "cs_mlp.cu"),
                os.path.join(CSRC, "cs_tc.cu"), os.path.join(CSRC, "cs_text.cu")]
-    deps = sources + [os.path.join(CSRC, "cs_kernels.cuh"), os.path.join(CSRC, "cs_umma.cuh"),
+    deps = sources + [os.path.join(CSRC, "cs_kernels.cuh"), os.path.join(CSRC, "cs_umma.cuh"), os.path.join(CSRC, "cs_fp64.cuh"),
                       os.path.join(CSRC, "cs_dtoa.h"), os.path.join(CSRC, "cs_text.h"),
                       os.path.join(ROOT, "include", "cs_gb300.h"), hdr]
     if not force and not _stale(LIB, deps):

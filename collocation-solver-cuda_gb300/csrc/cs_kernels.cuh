@@ -183,63 +183,6 @@ __device__ __forceinline__ void cs_static_for(F&& f) {
   }
 }
 
-// -x as an integer operation (the compiler spends an FP64 add on it)
-__device__ __forceinline__ double cs_neg(double x) {
-  return __hiloint2double(__double2hiint(x) ^ (int)0x80000000, __double2loint(x));
-}
-
-// 1 / p to the last bit or two: the reciprocal of the leading 23 bits in FP32,
-// then one third-order step r (1 + e + e^2), e = 1 - p r, |e| < 2^-22 (the
-// truncated geometric series for 1 / (1 - e)): 3 FP64 instructions where the
-// division takes about 9, on the unit that bounds these kernels.  Exponents
-// near the ends of the range (and 0, inf, NaN) divide.
-__device__ __forceinline__ double cs_rcp(double p) {
-  const int hi = __double2hiint(p), lo = __double2loint(p);
-  const int ex = (hi >> 20) & 0x7ff;
-  if (ex < 16 || ex > 2030) return 1.0 / p;
-  // mantissa in [1, 2) as FP32, its reciprocal in (1/2, 1]
-  const unsigned rf = __float_as_uint(__frcp_rn(__uint_as_float(0x3f800000u | ((unsigned)(hi & 0xfffff) << 3) | ((unsigned)lo >> 29))));
-  // the FP32 number as FP64 bits, scaled by 2^(1023 - ex), with p's sign
-  const int rex = (int)(rf >> 23) - 127 + 1023 + (1023 - ex);
-  const double r = __hiloint2double((hi & 0x80000000) | (rex << 20) | (int)((rf >> 3) & 0xfffff), (int)(rf << 29));
-  const double e = fma(-p, r, 1.0);
-  return fma(r, fma(e, e, e), r);
-}
-
-// 1 / sqrt(x), x > 0, to the last bit or two: FP32 on the leading bits, then
-// r (1 + h/2 + 3 h^2/8), h = 1 - x r^2, |h| < 2^-20 (the truncated binomial
-// series of (1 - h)^(-1/2)): 5 FP64 instructions in a chain
-__device__ __forceinline__ double cs_rsqrt(double x) {
-  const int hi = __double2hiint(x), lo = __double2loint(x);
-  const int ex = (hi >> 20) & 0x7ff;
-  if (hi < 0 || ex < 16 || ex > 2030) return 1.0 / sqrt(x);
-  const int odd = (ex & 1) ^ 1;  // 1023 is odd: mantissa 2^odd in [1, 4)
-  const float m = __uint_as_float(((unsigned)(127 + odd) << 23) | ((unsigned)(hi & 0xfffff) << 3) | ((unsigned)lo >> 29));
-  const unsigned rf = __float_as_uint(rsqrtf(m));
-  const int rex = (int)(rf >> 23) - 127 + 1023 - ((ex - 1023 - odd) >> 1);
-  const double r = __hiloint2double((rex << 20) | (int)((rf >> 3) & 0xfffff), (int)(rf << 29));
-  const double h = fma(-(x * r), r, 1.0);
-  return fma(r, h * fma(0.375, h, 0.5), r);
-}
-
-// Householder reflector H = I - t v v^T of a column with sum of squares ss and
-// leading entry x0: H column = g e_0 (the sign rule of
-// matrix_factorization_cuda.py:37-54), v_0 = x0 - g, v the column below, and
-// t = 2 / |v|^2 = 1 / (ss + |x0 g|).  False when |v|^2 < eps (nothing to
-// eliminate).  A square root and two divisions before: with few merges in
-// flight their latency (about 600 cycles each) was a third of a merge.
-__device__ __forceinline__ bool cs_reflector(double ss, double x0, double* g, double* v0, double* t) {
-  const double a = ss * cs_rsqrt(ss);
-  const double gg = (__double2hiint(x0) >= 0) ? cs_neg(a) : a;
-  const double half = fma(fabs(x0), a, ss);
-  *g = gg;
-  *v0 = x0 - gg;
-  *t = cs_rcp(half);
-  // half >= eps / 2, as integers (false for NaN)
-  const long long b = __double_as_longlong(half);
-  return b >= 0x3ca0000000000000ll && b <= 0x7ff0000000000000ll;
-}
-
 // Max of non-negative double bit patterns over the lanes of a warp that share
 // an instance, then one atomicMax per instance.  All 32 lanes must call it.
 __device__ __forceinline__ void cs_warp_max_atomic(unsigned long long* dst, int key, unsigned long long v, bool active) {
@@ -1609,47 +1552,44 @@ __device__ __forceinline__ constexpr bool cs_in_reflector(int k, int r) {
   return r == k || (r > k && !(L0 && r < CS_NY));
 }
 
-// column q (column c of the merge matrix) through the reflector (v below v0, t) of column k
+// x . q over the rows of reflector k (x: column k of the merge matrix, q:
+// column c), in two chains
 template <bool L0>
-__device__ __forceinline__ void cs_reflect(int k, int c, double v0, const double (&v)[2 * CS_NY], double t,
-                                           double (&q)[2 * CS_NY]) {
+__device__ __forceinline__ double cs_column_dot(int k, int c, const double (&x)[2 * CS_NY], const double (&q)[2 * CS_NY]) {
   const bool low0 = L0 && k == 0 && c >= CS_NY && c < 2 * CS_NY;       // zero below
   const bool unit0 = L0 && k == 0 && c >= 2 * CS_NY && c < 3 * CS_NY;  // zero above, unit below
-  double w0 = unit0 ? 0.0 : v0 * q[k], w1 = 0.0;
+  if (low0) return x[k] * q[k];
+  double a = 0.0, b = 0.0;
   if (unit0) {
 #pragma unroll
     for (int r = CS_NY; r < 2 * CS_NY; ++r)
-      if (r - CS_NY == c - 2 * CS_NY) w0 = v[r];
-  } else if (!low0) {
-    bool first = true;
-#pragma unroll
-    for (int r = k + 1; r < 2 * CS_NY; ++r)
-      if (cs_in_reflector<L0>(k, r)) {
-        if (((r - k) & 1) == 0) w0 = fma(v[r], q[r], w0);
-        else if (first) { w1 = v[r] * q[r]; first = false; }
-        else w1 = fma(v[r], q[r], w1);
-      }
+      if (r - CS_NY == c - 2 * CS_NY) a = x[r];
+    return a;
   }
-  const double bw = -t * (low0 || unit0 ? w0 : w0 + w1);
-  q[k] = unit0 ? bw * v0 : fma(bw, v0, q[k]);
-#pragma unroll
-  for (int r = k + 1; r < 2 * CS_NY; ++r)
-    if (cs_in_reflector<L0>(k, r)) q[r] = low0 ? bw * v[r] : fma(bw, v[r], q[r]);
-}
-
-// sum of squares of column q from row k
-template <bool L0>
-__device__ __forceinline__ double cs_column_ss(int k, const double (&q)[2 * CS_NY]) {
-  double a = q[k] * q[k], b = 0.0;
+  a = x[k] * q[k];
   bool first = true;
 #pragma unroll
   for (int r = k + 1; r < 2 * CS_NY; ++r)
     if (cs_in_reflector<L0>(k, r)) {
-      if (((r - k) & 1) == 0) a = fma(q[r], q[r], a);
-      else if (first) { b = q[r] * q[r]; first = false; }
-      else b = fma(q[r], q[r], b);
+      if (((r - k) & 1) == 0) a = fma(x[r], q[r], a);
+      else if (first) { b = x[r] * q[r]; first = false; }
+      else b = fma(x[r], q[r], b);
     }
   return a + b;
+}
+
+// column q (column c) through the reflector (v below v0, g, t) of column k;
+// p: the product of the untouched columns
+template <bool L0>
+__device__ __forceinline__ void cs_reflect(int k, int c, double p, double g, double v0, const double (&v)[2 * CS_NY],
+                                           double t, double (&q)[2 * CS_NY]) {
+  const bool low0 = L0 && k == 0 && c >= CS_NY && c < 2 * CS_NY;
+  const bool unit0 = L0 && k == 0 && c >= 2 * CS_NY && c < 3 * CS_NY;
+  const double bw = -t * (unit0 ? p : fma(-g, q[k], p));
+  q[k] = unit0 ? bw * v0 : fma(bw, v0, q[k]);
+#pragma unroll
+  for (int r = k + 1; r < 2 * CS_NY; ++r)
+    if (cs_in_reflector<L0>(k, r)) q[r] = low0 ? bw * v[r] : fma(bw, v[r], q[r]);
 }
 
 template <bool L0>
@@ -1661,9 +1601,9 @@ __device__ __forceinline__ void cs_merge_thread(const double* __restrict__ ra, c
 #pragma unroll
   for (int k = 0; k < CS_NY; ++k) {
     double g, v0, t;
-    if (cs_reflector(cs_column_ss<L0>(k, Q[k]), Q[k][k], &g, &v0, &t)) {
+    if (cs_reflector(cs_column_dot<L0>(k, k, Q[k], Q[k]), Q[k][k], &g, &v0, &t)) {
 #pragma unroll
-      for (int c = k + 1; c < CS_QC; ++c) cs_reflect<L0>(k, c, v0, Q[k], t, Q[c]);
+      for (int c = k + 1; c < CS_QC; ++c) cs_reflect<L0>(k, c, cs_column_dot<L0>(k, c, Q[k], Q[c]), g, v0, Q[k], t, Q[c]);
       Q[k][k] = g;
 #pragma unroll
       for (int r = k + 1; r < 2 * CS_NY; ++r) Q[k][r] = 0.0;
@@ -1731,38 +1671,32 @@ __device__ __forceinline__ void cs_merge_lanes(const double* __restrict__ ra, co
   cs_merge_column<L0>(ra, rb, c, Q);
 #pragma unroll
   for (int k = 0; k < CS_NY; ++k) {
-    // pivot lane k: the reflector of column k
-    double gk, v0k, tk;
-    // (the other lanes take 1: a zero column would send the warp through the
-    // out-of-range branches)
-    const double ss = cs_column_ss<L0>(k, Q);
-    const bool on = cs_reflector(c == k ? ss : 1.0, c == k ? Q[k] : 1.0, &gk, &v0k, &tk);
-    const double v0 = __shfl_sync(gm, v0k, k, CS_TL);
-    const double t = __shfl_sync(gm, tk, k, CS_TL);
-    const bool go = __shfl_sync(gm, (int)on, k, CS_TL) != 0;
+    // column k to every lane, its product with the lane's own; lane k's is the
+    // sum of squares, and every lane forms the reflector
     double v[2 * CS_NY];
 #pragma unroll
-    for (int r = k + 1; r < 2 * CS_NY; ++r)
+    for (int r = k; r < 2 * CS_NY; ++r)
       if (cs_in_reflector<L0>(k, r)) v[r] = __shfl_sync(gm, Q[r], k, CS_TL);
-    if (go) {
-      if (c > k) {
-        // (the general form: the lanes hold different columns)
-        double w0 = v0 * Q[k], w1 = 0.0;
-        bool first = true;
+    double p = v[k] * Q[k], p1 = 0.0;
+    bool first = true;
 #pragma unroll
-        for (int r = k + 1; r < 2 * CS_NY; ++r)
-          if (cs_in_reflector<L0>(k, r)) {
-            if (((r - k) & 1) == 0) w0 = fma(v[r], Q[r], w0);
-            else if (first) { w1 = v[r] * Q[r]; first = false; }
-            else w1 = fma(v[r], Q[r], w1);
-          }
-        const double bw = -t * (w0 + w1);
+    for (int r = k + 1; r < 2 * CS_NY; ++r)
+      if (cs_in_reflector<L0>(k, r)) {
+        if (((r - k) & 1) == 0) p = fma(v[r], Q[r], p);
+        else if (first) { p1 = v[r] * Q[r]; first = false; }
+        else p1 = fma(v[r], Q[r], p1);
+      }
+    p += p1;
+    double g, v0, t;
+    if (cs_reflector(__shfl_sync(gm, p, k, CS_TL), v[k], &g, &v0, &t)) {
+      if (c > k) {
+        const double bw = -t * fma(-g, Q[k], p);
         Q[k] = fma(bw, v0, Q[k]);
 #pragma unroll
         for (int r = k + 1; r < 2 * CS_NY; ++r)
           if (cs_in_reflector<L0>(k, r)) Q[r] = fma(bw, v[r], Q[r]);
       } else if (c == k) {
-        Q[k] = gk;
+        Q[k] = g;
 #pragma unroll
         for (int r = k + 1; r < 2 * CS_NY; ++r) Q[r] = 0.0;
       }
@@ -1959,24 +1893,17 @@ __device__ void cs_top_warp(const CsBatch& bt, int b, const double* row, double*
   double diag = 1.0;
   cs_static_for<0, CS_NT>([&](auto kc) {
     constexpr int k = decltype(kc)::value;
-    double s0 = q[k] * q[k], s1 = 0.0;
-    cs_static_for<k + 1, CS_NT>([&](auto rc) {
+    double v[CS_NT], p[2] = {0.0, 0.0};
+    cs_static_for<k, CS_NT>([&](auto rc) {
       constexpr int r = decltype(rc)::value;
-      if ((r - k) & 1) s1 = fma(q[r], q[r], s1); else s0 = fma(q[r], q[r], s0);
+      v[r] = __shfl_sync(full, q[r], k);
+      p[(r - k) & 1] = fma(v[r], q[r], p[(r - k) & 1]);
     });
-    double gk, v0k, tk;
-    const bool on = cs_reflector(c == k ? s0 + s1 : 1.0, c == k ? q[k] : 1.0, &gk, &v0k, &tk);
-    const double v0 = __shfl_sync(full, v0k, k), t = __shfl_sync(full, tk, k);
-    const bool go = __shfl_sync(full, (int)on, k) != 0;
+    p[0] += p[1];
+    double gk, v0, t;
+    const bool go = cs_reflector(__shfl_sync(full, p[0], k), v[k], &gk, &v0, &t);
     if (go) {
-      double w0 = v0 * q[k], w1 = 0.0;
-      double v[CS_NT];
-      cs_static_for<k + 1, CS_NT>([&](auto rc) {
-        constexpr int r = decltype(rc)::value;
-        v[r] = __shfl_sync(full, q[r], k);
-        if ((r - k) & 1) w1 = fma(v[r], q[r], w1); else w0 = fma(v[r], q[r], w0);
-      });
-      const double bw = (c > k) ? -t * (w0 + w1) : 0.0;
+      const double bw = (c > k) ? -t * fma(-gk, q[k], p[0]) : 0.0;
       q[k] = fma(bw, v0, q[k]);
       cs_static_for<k + 1, CS_NT>([&](auto rc) {
         constexpr int r = decltype(rc)::value;
