@@ -24,6 +24,7 @@
 #include "cs_gb300.h"
 
 int cs_internal_set_error(int code, const char* msg);
+int cs_internal_pool(cudaMemPool_t* out);
 
 namespace {
 
@@ -702,40 +703,6 @@ int noalloc_scratch(double** out) {
   return CS_OK;
 }
 
-// Pool of cs_babd_solve's scratch, one per device: stream-ordered, so calls on
-// any streams and threads may share it, and it keeps at most kPoolKeep bytes
-// between calls (more is given back at the next synchronisation).  cudaMalloc
-// and cudaFree around each call cost 0.2 ms, a third of a small solve.
-constexpr unsigned long long kPoolKeep = 64ull << 20;
-std::mutex g_pool_mu;
-cudaMemPool_t g_pool[128] = {nullptr};
-
-int scratch_pool(cudaMemPool_t* out) {
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return cs_internal_set_error(CS_ERR_CUDA, cudaGetErrorString(e));
-  if (dev < 0 || dev >= 128) return cs_internal_set_error(CS_ERR_CUDA, "cs_babd_solve: device index out of range");
-  std::lock_guard<std::mutex> lk(g_pool_mu);
-  if (!g_pool[dev]) {
-    cudaMemPoolProps props;
-    memset(&props, 0, sizeof(props));
-    props.allocType = cudaMemAllocationTypePinned;
-    props.location.type = cudaMemLocationTypeDevice;
-    props.location.id = dev;
-    cudaMemPool_t p = nullptr;
-    e = cudaMemPoolCreate(&p, &props);
-    unsigned long long keep = kPoolKeep;
-    if (e == cudaSuccess) e = cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep);
-    if (e != cudaSuccess) {
-      if (p) cudaMemPoolDestroy(p);
-      return cs_internal_set_error(CS_ERR_CUDA, cudaGetErrorString(e));
-    }
-    g_pool[dev] = p;
-  }
-  *out = g_pool[dev];
-  return CS_OK;
-}
-
 }  // namespace
 
 extern "C" int cs_babd_solve_noalloc(int ny, int np, int n, const double* A, const double* C, const double* H,
@@ -782,7 +749,7 @@ extern "C" int cs_babd_solve(int ny, int np, int n, const double* A, const doubl
   // scratch from the library's stream-ordered pool (element 0 carries the
   // singular flag)
   cudaMemPool_t pool = nullptr;
-  int rc = scratch_pool(&pool);
+  int rc = cs_internal_pool(&pool);
   if (rc != CS_OK) return rc;
   void* mem = nullptr;
   cudaError_t e = cudaMallocFromPoolAsync(&mem, (32 + scratch_doubles(d)) * sizeof(double), pool, st);

@@ -614,6 +614,7 @@ struct cs_mlp {
   std::vector<int> din, dout;  // per layer
   std::vector<long long> woff, boff;
   long long nparam = 0;
+  char* block = nullptr;  // the device memory of w .. pack
   float* w = nullptr;   // all weights and biases, FP32
   float* g = nullptr;   // gradients
   float* m1 = nullptr;  // Adam moments
@@ -883,16 +884,23 @@ extern "C" int cs_mlp_create(int n_in, int width, int depth, int n_out, unsigned
   std::vector<float> nrm(2 * (n_in + n_out));
   for (int c = 0; c < n_in; ++c) { nrm[c] = 0.f; nrm[n_in + c] = 1.f; }
   for (int c = 0; c < n_out; ++c) { nrm[2 * n_in + c] = 0.f; nrm[2 * n_in + n_out + c] = 1.f; }
+  // one block: parameters, gradients, Adam moments, normalisation, loss, packed
+  // weights
+  const size_t pb = (off * sizeof(float) + 255) / 256 * 256, nb = (nrm.size() * sizeof(float) + 255) / 256 * 256;
+  const size_t kb = M->fused ? net_pack_elems(M->net) * sizeof(__nv_bfloat16) : 0;
   if (cudaStreamCreateWithFlags(&M->st, cudaStreamNonBlocking) != cudaSuccess ||
-      cudaMalloc(&M->w, off * sizeof(float)) != cudaSuccess || cudaMalloc(&M->g, off * sizeof(float)) != cudaSuccess ||
-      cudaMalloc(&M->m1, off * sizeof(float)) != cudaSuccess || cudaMalloc(&M->m2, off * sizeof(float)) != cudaSuccess ||
-      cudaMalloc(&M->norm, nrm.size() * sizeof(float)) != cudaSuccess ||
-      cudaMalloc(&M->dloss, sizeof(double)) != cudaSuccess ||
-      (M->fused && (cudaMalloc(&M->pack, net_pack_elems(M->net) * sizeof(__nv_bfloat16)) != cudaSuccess ||
-                    cudaMemsetAsync(M->pack, 0, net_pack_elems(M->net) * sizeof(__nv_bfloat16), M->st) != cudaSuccess))) {
+      cudaMalloc(&M->block, 4 * pb + nb + 256 + kb) != cudaSuccess ||
+      (kb && cudaMemsetAsync(M->block + 4 * pb + nb + 256, 0, kb, M->st) != cudaSuccess)) {
     cs_mlp_free(M);
     return cs_internal_set_error(CS_ERR_NOMEM, "cs_mlp_create: device allocation failed");
   }
+  M->w = (float*)M->block;
+  M->g = (float*)(M->block + pb);
+  M->m1 = (float*)(M->block + 2 * pb);
+  M->m2 = (float*)(M->block + 3 * pb);
+  M->norm = (float*)(M->block + 4 * pb);
+  M->dloss = (double*)(M->block + 4 * pb + nb);
+  M->pack = (__nv_bfloat16*)(M->block + 4 * pb + nb + 256);
   cudaMemcpyAsync(M->w, hw.data(), off * sizeof(float), cudaMemcpyHostToDevice, M->st);
   cudaMemsetAsync(M->m1, 0, off * sizeof(float), M->st);
   cudaMemsetAsync(M->m2, 0, off * sizeof(float), M->st);
@@ -911,13 +919,7 @@ extern "C" void cs_mlp_free(cs_mlp* M) {
   mlp_free_acts(M);
   net_free(M);
   for (cs_mlp::Buf* b : {&M->in_x, &M->in_y, &M->in_perm, &M->out_y}) cudaFree(b->p);
-  cudaFree(M->pack);
-  cudaFree(M->w);
-  cudaFree(M->g);
-  cudaFree(M->m1);
-  cudaFree(M->m2);
-  cudaFree(M->norm);
-  cudaFree(M->dloss);
+  cudaFree(M->block);
   if (M->st) cudaStreamDestroy(M->st);
   delete M;
 }

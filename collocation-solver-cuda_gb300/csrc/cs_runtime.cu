@@ -313,6 +313,83 @@ __global__ void k_spares(int n, CsInst* inst, double alpha0, int* counts) {
 // error reporting for the other translation units of the library
 int cs_internal_set_error(int code, const char* msg) { return set_err(code, msg ? msg : ""); }
 
+// Device memory of the batches and of cs_babd_solve: one stream-ordered pool per
+// device, so calls on any streams and threads may share it.  It keeps at most
+// kPoolKeep bytes between uses; more goes back to the device at the next
+// synchronisation after it was freed.  A batch takes about fifty buffers and a
+// cudaMalloc / cudaFree pair costs 10 us and more, and cudaFree waits for the
+// whole device: half of the time of a small single solve.
+static const unsigned long long kPoolKeep = 256ull << 20;
+
+int cs_internal_pool(cudaMemPool_t* out) {
+  static std::mutex mu;
+  static cudaMemPool_t pools[128] = {nullptr};
+  int dev = 0;
+  CS_CUDA(cudaGetDevice(&dev));
+  if (dev < 0 || dev >= 128) return set_err(CS_ERR_CUDA, "device index out of range");
+  std::lock_guard<std::mutex> lk(mu);
+  if (!pools[dev]) {
+    cudaMemPoolProps props;
+    memset(&props, 0, sizeof(props));
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = dev;
+    cudaMemPool_t p = nullptr;
+    CS_CUDA(cudaMemPoolCreate(&p, &props));
+    unsigned long long keep = kPoolKeep;
+    const cudaError_t e = cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep);
+    if (e != cudaSuccess) {
+      cudaMemPoolDestroy(p);
+      return set_err(CS_ERR_CUDA, cudaGetErrorString(e));
+    }
+    pools[dev] = p;
+  }
+  *out = pools[dev];
+  return CS_OK;
+}
+
+// Page-locked words for the counts a solve reads back: slots of 64 bytes from
+// one page-locked block of the process (256 slots; beyond that each its own).
+struct HostSlots {
+  static const int kSlots = 256, kBytes = 64;
+  std::mutex mu;
+  char* base = nullptr;
+  std::vector<int> free_slots;
+};
+static HostSlots& host_slots() {
+  static HostSlots* h = new HostSlots();  // outlives every batch
+  return *h;
+}
+static int host_slot_take(int** out) {
+  HostSlots& h = host_slots();
+  {
+    std::lock_guard<std::mutex> lk(h.mu);
+    if (!h.base) {
+      CS_CUDA(cudaHostAlloc((void**)&h.base, (size_t)HostSlots::kSlots * HostSlots::kBytes, cudaHostAllocPortable));
+      for (int i = HostSlots::kSlots - 1; i >= 0; --i) h.free_slots.push_back(i);
+    }
+    if (!h.free_slots.empty()) {
+      *out = (int*)(h.base + (size_t)h.free_slots.back() * HostSlots::kBytes);
+      h.free_slots.pop_back();
+      return CS_OK;
+    }
+  }
+  CS_CUDA(cudaMallocHost((void**)out, HostSlots::kBytes));
+  return CS_OK;
+}
+static void host_slot_give(int* p) {
+  HostSlots& h = host_slots();
+  {
+    std::lock_guard<std::mutex> lk(h.mu);
+    const char* c = (const char*)p;
+    if (h.base && c >= h.base && c < h.base + (size_t)HostSlots::kSlots * HostSlots::kBytes) {
+      h.free_slots.push_back((int)((c - h.base) / HostSlots::kBytes));
+      return;
+    }
+  }
+  cudaFreeHost(p);
+}
+
 // ============================================================== module ===
 struct cs_module {
   int ny, nz, np, npe, nth, m, s, nrhs, cgw;
@@ -756,6 +833,7 @@ extern "C" void cs_opts_default(cs_opts* o) {
 struct DBuf {
   void* p = nullptr;
   size_t bytes = 0;
+  bool pooled = false;
 };
 
 struct cs_batch {
@@ -823,21 +901,33 @@ struct cs_batch {
   long long kind_launches[3] = {0, 0, 0};
 };
 
-static int dalloc(DBuf& b, size_t bytes) {
-  if (b.bytes >= bytes && b.p) return CS_OK;
-  if (b.p) cudaFree(b.p);
+// Grow-only buffer: from the pool, ordered on the batch's stream, or from
+// kPoolMax bytes on by cudaMalloc (there the mapping of the memory is what
+// costs, and the pool would map and unmap it for every batch: setting up a
+// 4 GB batch took 41.6 ms against 37.5).
+static const size_t kPoolMax = 256u << 10;
+
+static void dfree(cs_batch* bt, DBuf& b) {
+  if (b.p && b.pooled) cudaFreeAsync(b.p, bt->stream);
+  else if (b.p) cudaFree(b.p);
   b.p = nullptr;
   b.bytes = 0;
-  if (bytes == 0) bytes = 8;
-  CS_CUDA(cudaMalloc(&b.p, bytes));
-  b.bytes = bytes;
-  return CS_OK;
 }
 
-static void dfree(DBuf& b) {
-  if (b.p) cudaFree(b.p);
-  b.p = nullptr;
-  b.bytes = 0;
+static int dalloc(cs_batch* bt, DBuf& b, size_t bytes) {
+  if (b.bytes >= bytes && b.p) return CS_OK;
+  dfree(bt, b);
+  if (bytes == 0) bytes = 8;
+  b.pooled = bytes < kPoolMax;
+  if (b.pooled) {
+    cudaMemPool_t pool = nullptr;
+    CS_TRY(cs_internal_pool(&pool));
+    CS_CUDA(cudaMallocFromPoolAsync(&b.p, bytes, pool, bt->stream));
+  } else {
+    CS_CUDA(cudaMalloc(&b.p, bytes));
+  }
+  b.bytes = bytes;
+  return CS_OK;
 }
 
 static int alloc_slots(cs_batch* bt, long long cap, bool keep_current) {
@@ -846,25 +936,25 @@ static int alloc_slots(cs_batch* bt, long long cap, bool keep_current) {
   const size_t d = sizeof(double);
   for (int s = 0; s < 2; ++s) {
     if (keep_current && s == bt->cur) continue;
-    CS_TRY(dalloc(bt->t[s], c * d));
-    CS_TRY(dalloc(bt->y[s], c * M->ny * d));
-    CS_TRY(dalloc(bt->ydot[s], c * M->m * M->ny * d));
-    CS_TRY(dalloc(bt->zt[s], c * M->m * std::max(M->nz, 1) * d));
-    CS_TRY(dalloc(bt->znode[s], c * std::max(M->nz, 1) * d));
+    CS_TRY(dalloc(bt, bt->t[s], c * d));
+    CS_TRY(dalloc(bt, bt->y[s], c * M->ny * d));
+    CS_TRY(dalloc(bt, bt->ydot[s], c * M->m * M->ny * d));
+    CS_TRY(dalloc(bt, bt->zt[s], c * M->m * std::max(M->nz, 1) * d));
+    CS_TRY(dalloc(bt, bt->znode[s], c * std::max(M->nz, 1) * d));
   }
-  CS_TRY(dalloc(bt->inst_of, c * sizeof(int)));
-  CS_TRY(dalloc(bt->dy, c * M->ny * d));
-  CS_TRY(dalloc(bt->dydot, c * M->m * M->ny * d));
-  CS_TRY(dalloc(bt->dzt, c * M->m * std::max(M->nz, 1) * d));
-  CS_TRY(dalloc(bt->X, c * M->nrhs * M->s * d));
-  CS_TRY(dalloc(bt->rows0, c * M->rowsz * d));
-  CS_TRY(dalloc(bt->rows1, c * M->rowsz * d));
-  CS_TRY(dalloc(bt->tree, c * M->treesz * d));
-  CS_TRY(dalloc(bt->res, c * d));
-  CS_TRY(dalloc(bt->zform, c));
+  CS_TRY(dalloc(bt, bt->inst_of, c * sizeof(int)));
+  CS_TRY(dalloc(bt, bt->dy, c * M->ny * d));
+  CS_TRY(dalloc(bt, bt->dydot, c * M->m * M->ny * d));
+  CS_TRY(dalloc(bt, bt->dzt, c * M->m * std::max(M->nz, 1) * d));
+  CS_TRY(dalloc(bt, bt->X, c * M->nrhs * M->s * d));
+  CS_TRY(dalloc(bt, bt->rows0, c * M->rowsz * d));
+  CS_TRY(dalloc(bt, bt->rows1, c * M->rowsz * d));
+  CS_TRY(dalloc(bt, bt->tree, c * M->treesz * d));
+  CS_TRY(dalloc(bt, bt->res, c * d));
+  CS_TRY(dalloc(bt, bt->zform, c));
   if (M->prec_tree) {
-    CS_TRY(dalloc(bt->rows_keep, c * M->rowsz * d));
-    CS_TRY(dalloc(bt->dy_keep, c * M->ny * d));
+    CS_TRY(dalloc(bt, bt->rows_keep, c * M->rowsz * d));
+    CS_TRY(dalloc(bt, bt->dy_keep, c * M->ny * d));
   }
   bt->cap = (long long)c;
   return CS_OK;
@@ -885,10 +975,10 @@ static int grow_current(cs_batch* bt, long long need) {
               {&bt->inst_of, sizeof(int)}, {&bt->res, d}};
   for (auto& k : keep) {
     DBuf nb;
-    CS_TRY(dalloc(nb, (size_t)newcap * k.per));
+    CS_TRY(dalloc(bt, nb, (size_t)newcap * k.per));
     CS_CUDA(cudaMemcpyAsync(nb.p, k.b->p, (size_t)bt->T * k.per, cudaMemcpyDeviceToDevice, bt->stream));
     CS_CUDA(cudaStreamSynchronize(bt->stream));
-    dfree(*k.b);
+    dfree(bt, *k.b);
     *k.b = nb;
   }
   return alloc_slots(bt, newcap, true);
@@ -1195,22 +1285,22 @@ extern "C" int cs_batch_create(cs_module* M, int batch, long long node_capacity,
   }
   int rc = CS_OK;
   const size_t d = sizeof(double);
-  if ((rc = dalloc(bt->dN, batch * sizeof(int))) || (rc = dalloc(bt->doff, batch * sizeof(int))) ||
-      (rc = dalloc(bt->doff2, batch * sizeof(int))) || (rc = dalloc(bt->dp, batch * std::max(M->np, 1) * d)) ||
-      (rc = dalloc(bt->ddp, batch * std::max(M->np, 1) * d)) ||
-      (M->prec_tree && (rc = dalloc(bt->dp_keep, batch * std::max(M->np, 1) * d))) ||
-      (rc = dalloc(bt->dth, batch * std::max(M->nth, 1) * d)) || (rc = dalloc(bt->dinst, batch * sizeof(CsInst))) ||
-      (rc = dalloc(bt->dcounters, 64)) || (rc = dalloc(bt->l_act, batch * sizeof(int))) ||
-      (rc = dalloc(bt->dtrials, (size_t)batch * CS_LSW * sizeof(unsigned long long))) ||
-      (rc = dalloc(bt->l_jac, batch * sizeof(int))) || (rc = dalloc(bt->l_acc, batch * sizeof(int))) ||
-      (rc = dalloc(bt->l_seg, batch * sizeof(int))) || (rc = dalloc(bt->l_segp, (batch + 1) * sizeof(long long))) ||
-      (rc = dalloc(bt->l_actp, (batch + 1) * sizeof(long long))) ||
-      (rc = dalloc(bt->l_jacp, (batch + 1) * sizeof(long long))) ||
-      (rc = dalloc(bt->l_accp, (batch + 1) * sizeof(long long))) ||
-      (rc = dalloc(bt->l_lvlp, (size_t)CS_MAXLVL * (batch + 1) * sizeof(long long))) ||
-      (rc = dalloc(bt->l_n, 8 * sizeof(int))) ||
+  if ((rc = dalloc(bt, bt->dN, batch * sizeof(int))) || (rc = dalloc(bt, bt->doff, batch * sizeof(int))) ||
+      (rc = dalloc(bt, bt->doff2, batch * sizeof(int))) || (rc = dalloc(bt, bt->dp, batch * std::max(M->np, 1) * d)) ||
+      (rc = dalloc(bt, bt->ddp, batch * std::max(M->np, 1) * d)) ||
+      (M->prec_tree && (rc = dalloc(bt, bt->dp_keep, batch * std::max(M->np, 1) * d))) ||
+      (rc = dalloc(bt, bt->dth, batch * std::max(M->nth, 1) * d)) || (rc = dalloc(bt, bt->dinst, batch * sizeof(CsInst))) ||
+      (rc = dalloc(bt, bt->dcounters, 64)) || (rc = dalloc(bt, bt->l_act, batch * sizeof(int))) ||
+      (rc = dalloc(bt, bt->dtrials, (size_t)batch * CS_LSW * sizeof(unsigned long long))) ||
+      (rc = dalloc(bt, bt->l_jac, batch * sizeof(int))) || (rc = dalloc(bt, bt->l_acc, batch * sizeof(int))) ||
+      (rc = dalloc(bt, bt->l_seg, batch * sizeof(int))) || (rc = dalloc(bt, bt->l_segp, (batch + 1) * sizeof(long long))) ||
+      (rc = dalloc(bt, bt->l_actp, (batch + 1) * sizeof(long long))) ||
+      (rc = dalloc(bt, bt->l_jacp, (batch + 1) * sizeof(long long))) ||
+      (rc = dalloc(bt, bt->l_accp, (batch + 1) * sizeof(long long))) ||
+      (rc = dalloc(bt, bt->l_lvlp, (size_t)CS_MAXLVL * (batch + 1) * sizeof(long long))) ||
+      (rc = dalloc(bt, bt->l_n, 8 * sizeof(int))) ||
       (rc = alloc_slots(bt, std::max<long long>(node_capacity, 2 * batch), false)) ||
-      (M->big && (rc = dalloc(bt->wsp, (size_t)M->big_ctas * M->slab * d)))) {
+      (M->big && (rc = dalloc(bt, bt->wsp, (size_t)M->big_ctas * M->slab * d)))) {
     cs_batch_free(bt);
     return rc;
   }
@@ -1232,18 +1322,20 @@ extern "C" void cs_batch_free(cs_batch* bt) {
                  &bt->iN, &bt->ioff, &bt->it, &bt->iy, &bt->iz, &bt->ip, &bt->l_act, &bt->l_jac, &bt->l_acc,
                  &bt->l_actp, &bt->l_jacp, &bt->l_accp, &bt->l_seg, &bt->l_segp, &bt->l_lvlp, &bt->l_n, &bt->wsp,
                  &bt->rows_keep, &bt->dy_keep, &bt->dp_keep};
-  for (DBuf* b : all) dfree(*b);
+  for (DBuf* b : all) dfree(bt, *b);
   cs_text_scratch_free(&bt->text);
   for (int k = 0; k < 2; ++k)
     if (bt->graph[k]) cudaGraphExecDestroy(bt->graph[k]);
-  if (bt->h_n) cudaFreeHost(bt->h_n);
+  if (bt->h_n) host_slot_give(bt->h_n);
   for (auto& e : bt->ev_pool) {
     cudaEventDestroy(e.a);
     cudaEventDestroy(e.b);
   }
   for (int s = 0; s < 2; ++s) {
-    dfree(bt->t[s]); dfree(bt->y[s]); dfree(bt->ydot[s]); dfree(bt->zt[s]); dfree(bt->znode[s]);
+    for (DBuf* b : {&bt->t[s], &bt->y[s], &bt->ydot[s], &bt->zt[s], &bt->znode[s]}) dfree(bt, *b);
   }
+  // what the pool does not keep goes back to the device here
+  if (bt->stream) cudaStreamSynchronize(bt->stream);
   if (bt->own_stream && bt->stream) cudaStreamDestroy(bt->stream);
   delete bt;
 }
@@ -1285,12 +1377,12 @@ extern "C" int cs_batch_set_guess(cs_batch* bt, const int* N, const double* t, c
   if (M->np > 0) CS_CUDA(cudaMemcpyAsync(bt->dp.p, p, (size_t)bt->B * M->np * d, cudaMemcpyHostToDevice, st));
   if (M->nth > 0) CS_CUDA(cudaMemcpyAsync(bt->dth.p, theta, (size_t)bt->B * M->nth * d, cudaMemcpyHostToDevice, st));
   // device copy of the guess for cs_batch_reset
-  CS_TRY(dalloc(bt->iN, bt->B * sizeof(int)));
-  CS_TRY(dalloc(bt->ioff, bt->B * sizeof(int)));
-  CS_TRY(dalloc(bt->it, T * d));
-  CS_TRY(dalloc(bt->iy, T * M->ny * d));
-  CS_TRY(dalloc(bt->iz, T * std::max(M->nz, 1) * d));
-  CS_TRY(dalloc(bt->ip, (size_t)bt->B * std::max(M->np, 1) * d));
+  CS_TRY(dalloc(bt, bt->iN, bt->B * sizeof(int)));
+  CS_TRY(dalloc(bt, bt->ioff, bt->B * sizeof(int)));
+  CS_TRY(dalloc(bt, bt->it, T * d));
+  CS_TRY(dalloc(bt, bt->iy, T * M->ny * d));
+  CS_TRY(dalloc(bt, bt->iz, T * std::max(M->nz, 1) * d));
+  CS_TRY(dalloc(bt, bt->ip, (size_t)bt->B * std::max(M->np, 1) * d));
   CS_CUDA(cudaMemcpyAsync(bt->iN.p, bt->dN.p, bt->B * sizeof(int), cudaMemcpyDeviceToDevice, st));
   CS_CUDA(cudaMemcpyAsync(bt->ioff.p, bt->doff.p, bt->B * sizeof(int), cudaMemcpyDeviceToDevice, st));
   CS_CUDA(cudaMemcpyAsync(bt->it.p, bt->t[0].p, T * d, cudaMemcpyDeviceToDevice, st));
@@ -1406,14 +1498,19 @@ static int super_step(cs_batch* bt, const CsConsts& c, int nlvl) {
 
 // A CUDA graph of `reps` super-steps for the current layout (re-captured when
 // a remesh changes the buffers).
+static bool graph_valid(const cs_batch* bt, const CsBatchDev& v, const CsConsts& c, int nlvl) {
+  const int k = use_cta_path(bt) ? 1 : 0;
+  return bt->graph[k] && bt->graph_nlvl[k] == nlvl && bt->graph_tune[k] == bt->M->tune_ver &&
+         bt->graph_lo[k] == upper_levels(bt, nlvl) && bt->graph_refine[k] == bt->opts.refine &&
+         bt->graph_cap[k] == bt->work_cap && memcmp(&bt->graph_view[k], &v, sizeof(v)) == 0 &&
+         memcmp(&bt->graph_consts[k], &c, sizeof(c)) == 0;
+}
+
 static int get_graph(cs_batch* bt, const CsConsts& c, int nlvl, int reps) {
   const CsBatchDev v = devview(bt);
   const int k = use_cta_path(bt) ? 1 : 0;
   const int lo = upper_levels(bt, nlvl);
-  if (bt->graph[k] && bt->graph_nlvl[k] == nlvl && bt->graph_tune[k] == bt->M->tune_ver && bt->graph_lo[k] == lo &&
-      bt->graph_refine[k] == bt->opts.refine && bt->graph_cap[k] == bt->work_cap &&
-      memcmp(&bt->graph_view[k], &v, sizeof(v)) == 0 && memcmp(&bt->graph_consts[k], &c, sizeof(c)) == 0)
-    return CS_OK;
+  if (graph_valid(bt, v, c, nlvl)) return CS_OK;
   if (bt->graph[k]) {
     cudaGraphExecDestroy(bt->graph[k]);
     bt->graph[k] = nullptr;
@@ -1507,7 +1604,7 @@ extern "C" int cs_solve(cs_batch* bt, const cs_opts* opts) {
     s.alpha = o.alpha0;
   }
   CS_TRY(write_inst(bt, hi));
-  if (!bt->h_n) CS_CUDA(cudaMallocHost(&bt->h_n, 8 * sizeof(int)));
+  if (!bt->h_n) CS_TRY(host_slot_take(&bt->h_n));
   int rc = CS_OK;
   const long long max_super = 10000000;
   long long steps = 0;
@@ -1572,8 +1669,13 @@ extern "C" int cs_solve(cs_batch* bt, const cs_opts* opts) {
     const int nlvl = tree_levels(bt);
     CsBatchDev v0 = devview(bt);
     if ((rc = run_lists(bt, v0, 0, nlvl)) != CS_OK) break;
-    const bool use_graph = !bt->timing;
+    const long long direct_until = steps + 8;
     for (;;) {
+      // the first super-steps of a layout go out as launches: capturing and
+      // instantiating their graph costs more than it saves a solve that is done
+      // within a few (0.2 ms against 16 launches of 2 us per super-step, which
+      // the GPU hides)
+      const bool use_graph = !bt->timing && (steps >= direct_until || graph_valid(bt, devview(bt), c, nlvl));
       if (use_graph && (rc = get_graph(bt, c, nlvl, per_launch_steps)) != CS_OK) break;
       const bool cta = use_cta_path(bt);
       for (int k = 0; k < o.check_every && rc == CS_OK; ++k) {
@@ -1603,7 +1705,7 @@ extern "C" int cs_solve(cs_batch* bt, const cs_opts* opts) {
         rc = set_err(CS_ERR_STATE, "Newton phase did not terminate");
         break;
       }
-      if (use_graph && bt->h_n[0] <= cap_at && (bt->inst_cap == 0 || 2 * bt->h_n[0] <= bt->inst_cap)) {
+      if (!bt->timing && bt->h_n[0] <= cap_at && (bt->inst_cap == 0 || 2 * bt->h_n[0] <= bt->inst_cap)) {
         if ((rc = read_inst(bt, hi)) != CS_OK) break;
         set_cap(hi);
       }
@@ -1795,8 +1897,8 @@ extern "C" int cs_stage_residual(cs_batch* bt, double alpha, double* norms, doub
   cs_module* M = bt->M;
   CS_TRY(set_all_status(bt, ST_FRESH, alpha, 0));
   DBuf fa, fb;
-  if (f_a) CS_TRY(dalloc(fa, (size_t)bt->T * M->s * sizeof(double)));
-  if (f_b) CS_TRY(dalloc(fb, (size_t)bt->T * M->ny * sizeof(double)));
+  if (f_a) CS_TRY(dalloc(bt, fa, (size_t)bt->T * M->s * sizeof(double)));
+  if (f_b) CS_TRY(dalloc(bt, fb, (size_t)bt->T * M->ny * sizeof(double)));
   CsBatchDev v = devview(bt);
   v.fa_out = (double*)fa.p;
   v.fb_out = (double*)fb.p;
@@ -1818,8 +1920,8 @@ extern "C" int cs_stage_residual(cs_batch* bt, double alpha, double* norms, doub
     rc = set_err(CS_ERR_CUDA, "copy f_a");
   if (rc == CS_OK && f_b && cudaMemcpy(f_b, fb.p, (size_t)bt->T * M->ny * sizeof(double), cudaMemcpyDeviceToHost) != cudaSuccess)
     rc = set_err(CS_ERR_CUDA, "copy f_b");
-  dfree(fa);
-  dfree(fb);
+  dfree(bt, fa);
+  dfree(bt, fb);
   if (rc == CS_OK) {
     for (auto& s : hi) s.norm_bits = 0;
     rc = write_inst(bt, hi);
