@@ -1857,6 +1857,13 @@ extern "C" int cs_get_solution(cs_batch* bt, double* t, double* y, double* z, do
   return CS_OK;
 }
 
+// an instance's last slot holds no interval: its entries of a per-interval array
+// on the host are zero, not what the buffer held before
+static void clear_last(const cs_batch* bt, double* a, size_t per) {
+  if (!a || per == 0) return;
+  for (int b = 0; b < bt->B; ++b) memset(a + (size_t)(bt->hoff[b] + bt->hN[b] - 1) * per, 0, per * sizeof(double));
+}
+
 extern "C" int cs_get_state(cs_batch* bt, double* t, double* y, double* ydot, double* zt, double* z_nodes, double* p) {
   if (!bt || !bt->have_guess) return set_err(CS_ERR_STATE, "cs_get_state: no state");
   cs_module* M = bt->M;
@@ -1873,6 +1880,8 @@ extern "C" int cs_get_state(cs_batch* bt, double* t, double* y, double* ydot, do
   }
   if (p && M->np > 0) CS_CUDA(cudaMemcpyAsync(p, bt->dp.p, (size_t)bt->B * M->np * d, cudaMemcpyDeviceToHost, st));
   CS_CUDA(cudaStreamSynchronize(st));
+  clear_last(bt, ydot, (size_t)M->m * M->ny);
+  clear_last(bt, M->nz > 0 ? zt : nullptr, (size_t)M->m * M->nz);
   return CS_OK;
 }
 
@@ -1920,6 +1929,8 @@ extern "C" int cs_stage_residual(cs_batch* bt, double alpha, double* norms, doub
     rc = set_err(CS_ERR_CUDA, "copy f_a");
   if (rc == CS_OK && f_b && cudaMemcpy(f_b, fb.p, (size_t)bt->T * M->ny * sizeof(double), cudaMemcpyDeviceToHost) != cudaSuccess)
     rc = set_err(CS_ERR_CUDA, "copy f_b");
+  clear_last(bt, f_a, M->s);
+  clear_last(bt, f_b, M->ny);
   dfree(bt, fa);
   dfree(bt, fb);
   if (rc == CS_OK) {
@@ -1947,6 +1958,9 @@ extern "C" int cs_stage_newton_direction(cs_batch* bt, double alpha, double* row
   if (dzt && M->nz > 0) CS_CUDA(cudaMemcpyAsync(dzt, bt->dzt.p, (size_t)bt->T * M->m * M->nz * d, cudaMemcpyDeviceToHost, st));
   if (dp && M->np > 0) CS_CUDA(cudaMemcpyAsync(dp, bt->ddp.p, (size_t)bt->B * M->np * d, cudaMemcpyDeviceToHost, st));
   CS_CUDA(cudaStreamSynchronize(st));
+  clear_last(bt, rows, M->rowsz);
+  clear_last(bt, dydot, (size_t)M->m * M->ny);
+  clear_last(bt, M->nz > 0 ? dzt : nullptr, (size_t)M->m * M->nz);
   CS_TRY(check_config(bt));
   return set_all_status(bt, ST_FRESH, alpha, 0);
 }
