@@ -2043,6 +2043,7 @@ extern "C" __global__ void k_top(CsBatch bt) {
 #endif  // !CS_BIG_TREE
 
 // Back substitution of one tree level (top-down), warp per merge.
+#if !CS_BIG_TREE
 extern "C" __global__ void k_backsub_level(CsBatch bt, int l) {
 #if CS_TREE_THREAD
   {
@@ -2087,6 +2088,91 @@ extern "C" __global__ void k_backsub_level(CsBatch bt, int l) {
                     bt.dy + (size_t)(off + right) * CS_NY, bt.dp + (size_t)b * CS_NP, bt.dy + (size_t)(off + mid) * CS_NY);
   }
 }
+
+#else
+// Large blocks: a CTA of 256 threads per merge.  The products G y_l + E y_r + J p
+// are split over the columns (parts of the CTA), then the triangular solve goes
+// column by column with the next column already loaded.  (A warp per merge
+// walked 2 NY columns of 1 KB in a chain: 180 us for any level with few merges.)
+extern "C" __global__ void __launch_bounds__(256) k_backsub_level(CsBatch bt, int l) {
+  constexpr int NYR = (CS_NY + 31) / 32 * 32, PARTS = NYR >= 256 ? 1 : 256 / NYR, RPT = (CS_NY + 255) / 256;
+  constexpr int NC = 2 * CS_NY + CS_NPE;
+  constexpr bool XS = NC <= 2048;  // static shared memory stays below 48 KB
+  __shared__ double x[XS ? NC : 1], part[PARTS * NYR > 256 ? PARTS * NYR : 256], v[CS_NY], inv[CS_NY];
+  const int tid = threadIdx.x;
+  const int njac = bt.nlist[1];
+  const long long* pre = bt.lvl_pre + (size_t)l * (bt.B + 1);
+  const long long total = pre[njac];
+  for (long long it = blockIdx.x; it < total; it += gridDim.x) {
+    const int k = cs_find(pre, njac, it);
+    const int b = bt.jac[k];
+    const int mi = (int)(it - pre[k]);
+    const int n0 = bt.N[b] - 1;
+    if (mi >= (cs_rows_at(n0, l) >> 1)) continue;  // (uniform)
+    const int off = bt.off[b];
+    const int mid = (2 * mi + 1) << l, left = (2 * mi) << l, right = min((2 * mi + 2) << l, n0);
+    const double* rec = bt.tree + (size_t)(off + mid) * CS_TREESZ;
+    auto y_at = [&](int c) -> double {
+      return c < CS_NY ? bt.dy[(size_t)(off + left) * CS_NY + c]
+                       : (c < 2 * CS_NY ? bt.dy[(size_t)(off + right) * CS_NY + c - CS_NY]
+                                        : bt.dp[(size_t)b * CS_NP + c - 2 * CS_NY]);
+    };
+    if (XS)
+      for (int c = tid; c < NC; c += 256) x[c] = y_at(c);
+    auto xv = [&](int c) -> double { return XS ? x[c] : y_at(c); };
+    __syncthreads();
+#pragma unroll
+    for (int s = 0; s < RPT; ++s) {
+      const int a = (tid + 256 * s) % NYR, q = (tid + 256 * s) / NYR;
+      double u0 = 0.0, u1 = 0.0;
+      if (a < CS_NY && q < PARTS) {
+        int c = q;
+#pragma unroll 4
+        for (; c + PARTS < NC; c += 2 * PARTS) {
+          u0 = fma(rec[(size_t)(CS_NY + c) * CS_NY + a], xv(c), u0);
+          u1 = fma(rec[(size_t)(CS_NY + c + PARTS) * CS_NY + a], xv(c + PARTS), u1);
+        }
+        if (c < NC) u0 = fma(rec[(size_t)(CS_NY + c) * CS_NY + a], xv(c), u0);
+      }
+      if (q < PARTS) part[q * NYR + a] = u0 + u1;
+    }
+    __syncthreads();
+    for (int a = tid; a < CS_NY; a += 256) {
+      double s = rec[(size_t)(3 * CS_NY + CS_NPE) * CS_NY + a];
+#pragma unroll
+      for (int q = 0; q < PARTS; ++q) s -= part[q * NYR + a];
+      v[a] = s;
+      const double d = rec[(size_t)a * CS_NY + a];
+      inv[a] = d != 0.0 ? cs_rcp(d) : 0.0;
+    }
+    double nx[RPT];
+#pragma unroll
+    for (int s = 0; s < RPT; ++s)
+      nx[s] = (tid + 256 * s < CS_NY - 1) ? rec[(size_t)(CS_NY - 1) * CS_NY + tid + 256 * s] : 0.0;
+    __syncthreads();
+#pragma unroll 1
+    for (int r = CS_NY - 1; r >= 0; --r) {
+      const double xr = v[r] * inv[r];
+      double cu[RPT];
+#pragma unroll
+      for (int s = 0; s < RPT; ++s) {
+        cu[s] = nx[s];
+        nx[s] = (tid + 256 * s < r - 1) ? rec[(size_t)(r - 1) * CS_NY + tid + 256 * s] : 0.0;
+      }
+      __syncthreads();
+#pragma unroll
+      for (int s = 0; s < RPT; ++s) {
+        const int q = tid + 256 * s;
+        if (q < r) v[q] = fma(-cu[s], xr, v[q]);
+        if (q == r) v[r] = xr;
+      }
+      __syncthreads();
+    }
+    for (int a = tid; a < CS_NY; a += 256) bt.dy[(size_t)(off + mid) * CS_NY + a] = v[a];
+    __syncthreads();
+  }
+}
+#endif  // !CS_BIG_TREE
 
 #if !CS_BIG_TREE && CS_TREE_THREAD && CS_QC <= 32
 // The upper tree levels l >= l_first of every instance on the jac list (at most
@@ -2355,8 +2441,10 @@ extern "C" __global__ void k_babd_cta(CsBatch bt) {}
 //                 cs_condense_tc, FP32 storage and the block updates on
 //                 the tensor cores with tcgen05.
 //   k_tree_level  one CTA per merge, compact-WY Householder in panels of
-//                 CS_HB reflectors (CS_PREC_TREE: on the tensor cores).
-//   k_top         one CTA per instance.
+//                 CS_HQ (CS_PREC_TREE: CS_HB, on the tensor cores)
+//                 reflectors; a cluster of CTAs per merge where a
+//                 level has few.
+//   k_top         one CTA or cluster per instance.
 #define CS_NB 16
 #define CS_LDG (((CS_NCOL1 + 3) / 4) * 4)   // row stride of the slab matrix
 #define CS_PLD (CS_NB + 1)                  // row stride of the panel (shared)
@@ -2370,14 +2458,22 @@ extern "C" __global__ void k_babd_cta(CsBatch bt) {}
 #define CS_QSZ (CS_QLD * CS_QC)
 #define CS_TSZ (CS_TLD * (CS_NT + 1))
 #define CS_DRSZ ((CS_NY + CS_NP) * (2 * CS_NY + CS_NP))
-// merges: Householder panels of CS_HB reflectors; shared: V [HB][QLD] | T [HB][HB] | G [HB][HB] | tau [HB] | red [32]
+// merges and top system: Householder panels of CS_HQ reflectors (cs_qr_blocked);
+// shared: V [HQ][ld] | V_j . V_i [HQ][HQ] | tau [HQ] | red [8][HQ] | row [HQ] |
+// bw [HQ] | header [HQ]; the matrix in the slab; the diagonal blocks of R
+// [npiv][HQ] in the slab of each CTA (a panel is still read by other CTAs when
+// they are done)
+#define CS_HQ 8
+#define CS_SM_QR(ld) (CS_HQ * (ld) + CS_HQ * CS_HQ + 12 * CS_HQ)
+#define CS_SM_HB CS_SM_QR(CS_QLD)
+// threads of a merge: a row of a panel each, and a warp for each block of columns
+// that falls to one of eight CTAs
+#define CS_TREE_TB (CS_PREC_TREE ? 256 : (CS_NY <= 32 ? 64 : (CS_NY <= 64 ? 128 : 256)))
+#define CS_TQ_SMEM ((long long)CS_SM_QR(CS_TLD) * 8 <= CS_SMEM_MAX)
+#define CS_WS_TREE ((long long)CS_QSZ + CS_HQ * CS_NY)
+#define CS_WS_TOP ((long long)CS_TSZ + (long long)CS_DRSZ + (CS_HQ + 2) * CS_NT + (CS_TQ_SMEM ? 0 : CS_SM_QR(CS_TLD)))
+#define CS_SM_TREE (CS_SM_HB)
 #define CS_HB 16
-#define CS_SM_HB (CS_HB * CS_QLD + 2 * CS_HB * CS_HB + CS_HB + 32)
-#define CS_Q_SMEM (((long long)CS_QSZ + CS_SM_HB) * 8 <= CS_SMEM_MAX)
-#define CS_T_SMEM (((long long)CS_TSZ + 32) * 8 <= CS_SMEM_MAX)
-#define CS_WS_TREE (CS_Q_SMEM ? 0ll : (long long)CS_QSZ)
-#define CS_WS_TOP ((CS_T_SMEM ? 0ll : (long long)CS_TSZ) + (long long)CS_DRSZ)
-#define CS_SM_TREE ((CS_Q_SMEM ? CS_QSZ : 0) + CS_SM_HB)
 // reduced precision (CS_PREC_TREE != 0): FP32 merge matrix; shared floats V [HB][QLD] |
 // T, G [HB][HB] | tau [HB] | W [QC][HB], then red [32] doubles
 #define CS_SHF (CS_HB * CS_QLD + 2 * CS_HB * CS_HB + CS_HB + CS_QC * CS_HB)
@@ -2386,7 +2482,7 @@ extern "C" __global__ void k_babd_cta(CsBatch bt) {}
 #define CS_Q_SMEM_LP (((long long)CS_QSZ_LP + CS_SM_HB_LP) * 8 <= CS_SMEM_MAX)
 #define CS_WS_TREE_LP (CS_Q_SMEM_LP ? 0ll : (long long)CS_QSZ_LP)
 #define CS_SM_TREE_LP ((CS_Q_SMEM_LP ? CS_QSZ_LP : 0) + CS_SM_HB_LP)
-#define CS_SM_TOP ((CS_T_SMEM ? CS_TSZ : 0) + 32)
+#define CS_SM_TOP (CS_TQ_SMEM ? CS_SM_QR(CS_TLD) : 0)
 
 // tensor-core operands: FP32 rounded to TF32 (round to nearest, ties away),
 // or two FP32 rounded to a BF16 pair (lo in the low half)
@@ -2407,12 +2503,13 @@ __device__ __forceinline__ unsigned cs_dyn_smem_bytes() {
   return r;
 }
 
-// the launch gives this CTA a slab of at least `slab` doubles and `sm`
+// the launch gives this CTA (last: the last CTA of its cluster, so that a
+// cluster decides as one) a slab of at least `slab` doubles and `sm`
 // doubles of shared memory; otherwise count a configuration error and do
 // nothing (the host reports it)
-__device__ __forceinline__ bool cs_big_ok(const CsBatch& bt, long long slab, long long sm) {
+__device__ __forceinline__ bool cs_big_ok(const CsBatch& bt, long long slab, long long sm, int last) {
   const bool ok = blockDim.x <= 256 && (blockDim.x & 31) == 0 && (long long)cs_dyn_smem_bytes() >= sm * 8 &&
-                  (slab == 0 || (bt.wsp != nullptr && (int)blockIdx.x < bt.wsp_ctas && bt.wsp_stride >= slab));
+                  (slab == 0 || (bt.wsp != nullptr && last < bt.wsp_ctas && bt.wsp_stride >= slab));
   if (!ok && threadIdx.x == 0) atomicAdd(&bt.counters[7], 1ull);
   return ok;
 }
@@ -2438,17 +2535,6 @@ __device__ __forceinline__ void cs_cta_argmax(unsigned long long& best, int& bro
     if (ob > best || (ob == best && orow < brow)) { best = ob; brow = orow; }
   }
   __syncthreads();
-}
-
-// sum over the CTA; every thread gets the same value (red: 8 doubles)
-__device__ __forceinline__ double cs_cta_sum(double v, double* red) {
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
-  __syncthreads();
-  double s = 0.0;
-  for (int w = 0; w < (int)(blockDim.x >> 5); ++w) s += red[w];
-  __syncthreads();
-  return s;
 }
 
 #if CS_BIG_COND
@@ -3182,9 +3268,9 @@ __device__ bool cs_condense_tc(const CsBatch& bt, int slot, double* slab, unsign
 extern "C" __global__ void __launch_bounds__(256, 2) k_condense(CsBatch bt) {
   extern __shared__ __align__(128) double smem[];
 #if CS_PREC == 0
-  if (!cs_big_ok(bt, CS_WS_COND, CS_SM_COND)) return;
+  if (!cs_big_ok(bt, CS_WS_COND, CS_SM_COND, blockIdx.x)) return;
 #else
-  if (!cs_big_ok(bt, CS_WS_COND, CS_TC_SMD)) return;
+  if (!cs_big_ok(bt, CS_WS_COND, CS_TC_SMD, blockIdx.x)) return;
   // the CTA's tensor-memory accumulator and MMA barrier, for all its intervals
   unsigned char* smb = reinterpret_cast<unsigned char*>(smem);
   unsigned long long* mb = reinterpret_cast<unsigned long long*>(smb + CS_TC_MISC);
@@ -3230,180 +3316,281 @@ extern "C" __global__ void __launch_bounds__(256, 2) k_condense(CsBatch bt) {
 #endif  // CS_BIG_COND
 
 #if CS_BIG_TREE
-// Householder column k of a column-major matrix A (leading dimension ld,
-// rows k..n-1) applied to columns k+1..nc-1, CTA-wide: a warp per column,
-// lanes over rows.  Sign rule and early skip as matrix_factorization_cuda.py:37-54.
-__device__ __forceinline__ void cs_householder_cta(double* A, int ld, int n, int nc, int k, double* red) {
-  const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, w = tid >> 5, nw = nt >> 5;
-  const double* vk = A + (size_t)k * ld;
-  double ss = 0.0;
-  for (int r = k + tid; r < n; r += nt) ss += vk[r] * vk[r];
-  ss = cs_cta_sum(ss, red);
-  const double x0 = vk[k];
-  const double sgn = (x0 >= 0.0) ? 1.0 : -1.0;
-  const double g = -sgn * sqrt(ss);
-  const double v0 = x0 - g;
-  const double vs = ss - x0 * x0 + v0 * v0;
-  if (vs < CS_EPS) return;  // uniform: nothing to eliminate in this column
-  const double beta = -2.0 / vs;
-  for (int c = k + 1 + w; c < nc; c += nw) {
-    double* col = A + (size_t)c * ld;
-    double wv = (lane == 0) ? v0 * col[k] : 0.0;
-    for (int r = k + 1 + lane; r < n; r += 32) wv = fma(vk[r], col[r], wv);
-    for (int o = 16; o > 0; o >>= 1) wv += __shfl_xor_sync(0xffffffffu, wv, o);
-    const double bw = beta * wv;
-    if (lane == 0) col[k] = fma(bw, v0, col[k]);
-    for (int r = k + 1 + lane; r < n; r += 32) col[r] = fma(bw, vk[r], col[r]);
+// ---- clusters: a merge (or top system) may be shared by the CTAs of a cluster
+__device__ __forceinline__ unsigned cs_cluster_rank() {
+  unsigned r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ unsigned cs_cluster_size() {
+  unsigned r;
+  asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
+  return r;
+}
+// barrier of the cluster (of the CTA when it is alone); orders memory
+__device__ __forceinline__ void cs_cluster_sync(int G) {
+  if (G > 1) {
+    __threadfence();
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+  } else {
+    __syncthreads();
   }
-  __syncthreads();
-  double* ck = A + (size_t)k * ld;
-  if (tid == 0) ck[k] = g;
-  for (int r = k + 1 + tid; r < n; r += nt) ck[r] = 0.0;
-  __syncthreads();
 }
 
-// Merge of block rows a and b, one CTA (layout as cs_merge_warp), blocked
-// Householder (compact WY, as LAPACK's geqrt): each panel of CS_HB columns is
-// factorised column by column (cs_householder_cta restricted to the panel),
-// its reflectors H_i = I - tau_i v_i v_i^T (tau = 2/|v|^2, the sign rule of
-// matrix_factorization_cuda.py:37-54) are accumulated as
-// H_1 ... H_kb = I - V T V^T, and the columns right of the panel are updated
-// at once, C <- C - V (T^T (V^T C)), one thread per column.
-__device__ void cs_merge_cta(const double* ra, const double* rb, double* out_row, double* rec, double* Q, double* sh) {
-  const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, w = tid >> 5, nw = nt >> 5;
-  constexpr int n = 2 * CS_NY;
-  double* V = sh;                          // [HB][QLD] column-major, zero above row k0 + i
-  double* Tm = V + CS_HB * CS_QLD;         // [HB][HB], T[j][i] at Tm[i * HB + j]
-  double* G = Tm + CS_HB * CS_HB;          // [HB][HB], V_j . V_i at G[i * HB + j]
-  double* tau = G + CS_HB * CS_HB;         // [HB]
-  double* red = tau + CS_HB;               // [32]
+// Blocked Householder QR (compact WY) of the first npiv columns of a
+// column-major matrix Q (n rows, ncol columns, leading dimension LD), applied
+// to the others; sign rule and early skip as matrix_factorization_cuda.py:37-54.
+// One CTA, or the G CTAs of a cluster.
+//
+// Panels of CS_HQ columns, a row per thread with the panel's columns in
+// registers: per column one pass forms the products of the column with all the
+// panel's columns (its own: the sum of squares; the finished reflectors: the
+// v_j . v of the WY form), reduced over the warp by halving (9 adds instead of
+// 40), two barriers.  Every CTA of a cluster factors the panel for itself (it
+// is a latency chain: sharing it would cost a cluster barrier per column).  The
+// columns right of the panel are dealt out in blocks of eight, block b to CTA
+// b % G: C <- C - V T^T (V^T C), four lanes per column.  Panels of 8: with 16 the
+// panel and the T solves took a quarter of the FP64 instructions at 32-entry
+// blocks (a tree of 256 x 256 merges 53.9 ms against 45.9).
+//
+// What bounds it is the SM's FP64 unit (16 cycles per warp instruction).  Upper
+// tree levels have fewer merges than the GPU has SMs: a 256 x 449 merge takes
+// one SM 5.3 ms, eight 1.1.  Tree of the K = 32 chain (1,024 intervals, ny 128):
+// 88 -> 39 ms, of the K = 16 one 25 -> 13; top system (column by column by one
+// CTA before) 20 -> 2.8 and 2.4 -> 0.9 ms.
+//
+// l0 > 0: the pivot columns are l0 unit vectors over a block of l0 rows (C = I,
+// block rows as condensed): a panel's reflectors are zero between the panel's
+// own rows and that block, and those rows are left out (28 % of the work).
+//
+// R's diagonal blocks end up in Rd [npiv][CS_HQ] of every CTA (entry (row k0 +
+// i, column c) at c * HB + i), its other entries and the transformed columns in Q.
+// maximum rows NR (compile time: rows per thread).
+struct CsQrRows {
+  int k0, na, rb;  // rows k0 .. k0 + na - 1, then rb ..
+  __device__ __forceinline__ int at(int i) const { return i < na ? k0 + i : rb + (i - na); }
+};
+
+template <int NR, int LD, int TB>
+__device__ void cs_qr_blocked(double* Q, int n, int ncol, int npiv, int l0, int rank, int G, double* sh, double* Rd) {
+  constexpr int HB = CS_HQ, RPT = (NR + TB - 1) / TB;
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, nw = TB / 32;
+  double* V = sh;                 // [HB][LD], compact rows
+  double* Gm = V + HB * LD;       // v_j . v_i (j < i) at i * HB + j
+  double* tau = Gm + HB * HB;
+  double* red = tau + HB;         // [8][HB]
+  double* rowk = red + 8 * HB;
+  double* bw = rowk + HB;
+  double* hdr = bw + HB;          // v0, on
+#pragma unroll 1
+  for (int k0 = 0; k0 < npiv; k0 += HB) {
+    const int kb = min(HB, npiv - k0), pe = k0 + kb;
+    CsQrRows rows;
+    rows.k0 = k0;
+    rows.na = l0 ? kb : n - k0;
+    rows.rb = l0;
+    const int nr = l0 ? kb + (n - l0) : n - k0;
+    const int pw = min(nw, (nr + 31) >> 5);  // warps with panel rows
+    double a[RPT][HB];
+#pragma unroll
+    for (int s = 0; s < RPT; ++s) {
+      const int i = tid + TB * s;
+      const bool in = i < nr;
+      const double* src = Q + (size_t)k0 * LD + (in ? rows.at(i) : 0);
+#pragma unroll
+      for (int c = 0; c < HB; ++c) a[s][c] = (in && c < kb) ? (G > 1 ? __ldcg(src + (size_t)c * LD) : src[(size_t)c * LD]) : 0.0;
+    }
+    cs_static_for<0, HB>([&](auto kc) {
+      constexpr int kk = decltype(kc)::value;
+      if (kk < kb) {
+        // products of column kk (rows from kk on) with the panel's columns
+        if (w < pw) {
+          double p[HB];
+#pragma unroll
+          for (int c = 0; c < HB; ++c) p[c] = 0.0;
+#pragma unroll
+          for (int s = 0; s < RPT; ++s) {
+            const double x = (s > 0 || tid >= kk) ? a[s][kk] : 0.0;
+#pragma unroll
+            for (int c = 0; c < HB; ++c) p[c] = fma(x, a[s][c], p[c]);
+          }
+          if (tid == kk) {
+#pragma unroll
+            for (int c = 0; c < HB; ++c) rowk[c] = a[0][c];
+          }
+          // sums over the warp by halving: 32 / HB neighbouring lanes end with
+          // a column's
+#pragma unroll
+          for (int h = HB / 2; h >= 1; h >>= 1) {
+            const bool up = (lane & (32 / HB * h)) != 0;
+#pragma unroll
+            for (int c = 0; c < HB; ++c)
+              if (c < h) {
+                const double give = up ? p[c] : p[c + h], keep = up ? p[c + h] : p[c];
+                p[c] = keep + __shfl_xor_sync(0xffffffffu, give, 32 / HB * h);
+              }
+          }
+#pragma unroll
+          for (int o = 16 / HB; o >= 1; o >>= 1) p[0] += __shfl_xor_sync(0xffffffffu, p[0], o);
+          if (lane % (32 / HB) == 0) red[w * HB + lane / (32 / HB)] = p[0];
+        }
+        __syncthreads();
+        if (w == 0) {
+          const int c = lane & (HB - 1);
+          double p = 0.0, q = 0.0;
+          for (int u = 0; u < pw; u += 2) {
+            p += red[u * HB + c];
+            if (u + 1 < pw) q += red[(u + 1) * HB + c];
+          }
+          p += q;
+          double g, v0, t;
+          const bool on = cs_reflector(__shfl_sync(0xffffffffu, p, kk), rowk[kk], &g, &v0, &t);
+          const double d = fma(-g, rowk[c], p);  // v . column c
+          if (lane < HB) {
+            if (c > kk) bw[c] = on ? -t * d : 0.0;
+            else if (c < kk) Gm[kk * HB + c] = on ? d : 0.0;
+            else {
+              tau[kk] = on ? t : 0.0;
+              hdr[0] = on ? v0 : 0.0;
+              hdr[1] = on ? g : rowk[kk];
+              hdr[2] = on ? 1.0 : 0.0;
+            }
+          }
+        }
+        __syncthreads();
+        if (w < pw) {
+          const bool on = hdr[2] != 0.0;
+          const double v0 = hdr[0], g = hdr[1];
+#pragma unroll
+          for (int s = 0; s < RPT; ++s) {
+            const int i = tid + TB * s;
+            const double v = (!on || (s == 0 && tid < kk)) ? 0.0 : ((s == 0 && tid == kk) ? v0 : a[s][kk]);
+#pragma unroll
+            for (int c = kk + 1; c < HB; ++c) a[s][c] = fma(bw[c], v, a[s][c]);
+            if (s == 0 && tid == kk) {
+              // row k0 + kk of R
+              Rd[(size_t)(k0 + kk) * HB + kk] = g;
+#pragma unroll
+              for (int c = kk + 1; c < HB; ++c)
+                if (c < kb) Rd[(size_t)(k0 + c) * HB + kk] = a[0][c];
+            }
+            a[s][kk] = v;
+            if (i < nr) V[kk * LD + i] = v;
+          }
+        }
+      }
+    });
+    // T = (diag(1 / tau) + U)^-1, U the products v_i . v_j above the diagonal: a
+    // column per lane by back substitution, stored in place as T^T (lower).  A
+    // last panel narrower than CS_HQ: its unused reflectors are the identity
+    for (int e = tid; e < (HB - kb) * nr; e += TB) V[(kb + e / nr) * LD + e % nr] = 0.0;
+    if (w == 0) {
+      const int c = lane & (HB - 1);
+      double t[HB];
+#pragma unroll
+      for (int i = 0; i < HB; ++i) t[i] = i == c ? 1.0 : 0.0;
+#pragma unroll
+      for (int i = HB - 1; i >= 0; --i) {
+        t[i] = i < kb ? t[i] * tau[i] : 0.0;
+#pragma unroll
+        for (int j = 0; j < i; ++j) t[j] = fma(i < kb ? -Gm[i * HB + j] : 0.0, t[i], t[j]);
+      }
+      __syncwarp();
+      if (lane < HB) {
+#pragma unroll
+        for (int i = 0; i < HB; ++i) Gm[c * HB + i] = t[i];
+      }
+    }
+    __syncthreads();
+    // columns right of the panel, blocks of eight
+    const int nblk = (ncol + 7) >> 3;
+    int b0 = pe >> 3;
+    b0 += ((rank - b0) % G + G) % G;
+    for (int blk = b0 + G * w; blk < nblk; blk += G * nw) {
+      const int c = blk * 8 + (lane >> 2), part = lane & 3;
+      const bool act = c < ncol && c >= pe;
+      double* col = Q + (size_t)c * LD;
+      double wv[HB];
+#pragma unroll
+      for (int i = 0; i < HB; ++i) wv[i] = 0.0;
+      if (act) {
+#pragma unroll 4
+        for (int i = part; i < nr; i += 4) {
+          const double x = col[rows.at(i)];
+#pragma unroll
+          for (int j = 0; j < HB; ++j) wv[j] = fma(V[j * LD + i], x, wv[j]);
+        }
+      }
+      __syncwarp();
+      // sums over the column's four lanes by halving (lane q ends with entries
+      // 4 q ..), spread again; entries part, part + 4, .. of w' = T^T w, spread
+      // (48 FP64 instructions; 168 with every lane adding and solving for all)
+#pragma unroll
+      for (int h = HB / 2; h >= HB / 4; h >>= 1) {
+        const bool up = (part & (h * 4 / HB)) != 0;
+#pragma unroll
+        for (int i = 0; i < HB; ++i)
+          if (i < h) {
+            const double give = up ? wv[i] : wv[i + h], keep = up ? wv[i + h] : wv[i];
+            wv[i] = keep + __shfl_xor_sync(0xffffffffu, give, h * 4 / HB);
+          }
+      }
+      double wf[HB], u[HB / 4];
+#pragma unroll
+      for (int i = 0; i < HB; ++i) wf[i] = __shfl_sync(0xffffffffu, wv[i % (HB / 4)], i / (HB / 4), 4);
+#pragma unroll
+      for (int q = 0; q < HB / 4; ++q) {
+        u[q] = 0.0;
+#pragma unroll
+        for (int j = 0; j < 4 * q + 4; ++j) u[q] = fma(Gm[(part + 4 * q) * HB + j], wf[j], u[q]);
+      }
+#pragma unroll
+      for (int i = 0; i < HB; ++i) wv[i] = __shfl_sync(0xffffffffu, u[i >> 2], i & 3, 4);
+      if (act) {
+#pragma unroll 4
+        for (int i = part; i < nr; i += 4) {
+          double* e = col + rows.at(i);
+          double x = *e;
+#pragma unroll
+          for (int j = 0; j < HB; ++j) x = fma(-V[j * LD + i], wv[j], x);
+          *e = x;
+        }
+      }
+    }
+    cs_cluster_sync(G);
+  }
+}
+
+// Merge of block rows a and b (layout as cs_merge_warp) by a CTA or a cluster;
+// columns in blocks of eight, dealt out as in cs_qr_blocked.
+__device__ void cs_merge_cta(const double* ra, const double* rb, double* out_row, double* rec, double* Q, double* sh,
+                             double* Rd, bool level0, int rank, int G) {
+  const int tid = threadIdx.x, nt = blockDim.x;
   for (int e = tid; e < CS_QC * CS_NY; e += nt) {
     const int c = e / CS_NY, r = e - c * CS_NY;
+    if (((c >> 3) % G) != rank) continue;
     double top, bot;
-    if (c < CS_NY) { top = ra[(CS_NY + c) * CS_NY + r]; bot = rb[c * CS_NY + r]; }
+    if (c < CS_NY) { top = level0 ? (r == c ? 1.0 : 0.0) : ra[(CS_NY + c) * CS_NY + r]; bot = rb[c * CS_NY + r]; }
     else if (c < 2 * CS_NY) { top = ra[(c - CS_NY) * CS_NY + r]; bot = 0.0; }
-    else if (c < 3 * CS_NY) { top = 0.0; bot = rb[(CS_NY + c - 2 * CS_NY) * CS_NY + r]; }
+    else if (c < 3 * CS_NY) { top = 0.0; bot = level0 ? (r == c - 2 * CS_NY ? 1.0 : 0.0) : rb[(CS_NY + c - 2 * CS_NY) * CS_NY + r]; }
     else if (c < 3 * CS_NY + CS_NPE) { top = ra[(2 * CS_NY + c - 3 * CS_NY) * CS_NY + r]; bot = rb[(2 * CS_NY + c - 3 * CS_NY) * CS_NY + r]; }
     else { top = ra[(2 * CS_NY + CS_NPE) * CS_NY + r]; bot = rb[(2 * CS_NY + CS_NPE) * CS_NY + r]; }
     Q[(size_t)c * CS_QLD + r] = top;
     Q[(size_t)c * CS_QLD + CS_NY + r] = bot;
   }
-  __syncthreads();
-#pragma unroll 1
-  for (int k0 = 0; k0 < CS_NY; k0 += CS_HB) {
-    const int kb = min(CS_HB, CS_NY - k0);
-    const int pe = k0 + kb;  // panel end (exclusive)
-    // ---- panel: reflectors of columns k0 .. pe-1, applied inside the panel
-#pragma unroll 1
-    for (int kk = 0; kk < kb; ++kk) {
-      const int k = k0 + kk;
-      double* vk = Q + (size_t)k * CS_QLD;
-      double ss = 0.0;
-      for (int r = k + tid; r < n; r += nt) ss += vk[r] * vk[r];
-      ss = cs_cta_sum(ss, red);
-      const double x0 = vk[k];
-      const double g = (x0 >= 0.0) ? -sqrt(ss) : sqrt(ss);
-      const double v0 = x0 - g;
-      const double vs = ss - x0 * x0 + v0 * v0;
-      double* Vi = V + kk * CS_QLD;
-      if (vs < CS_EPS) {  // uniform: nothing to eliminate, H = I
-        for (int r = tid; r < n; r += nt) Vi[r] = 0.0;
-        if (tid == 0) tau[kk] = 0.0;
-        __syncthreads();
-        continue;
-      }
-      const double beta = -2.0 / vs;
-      for (int r = tid; r < n; r += nt) Vi[r] = (r < k) ? 0.0 : ((r == k) ? v0 : vk[r]);
-      if (tid == 0) tau[kk] = 2.0 / vs;
-      for (int c = k + 1 + w; c < pe; c += nw) {
-        double* col = Q + (size_t)c * CS_QLD;
-        double wv = (lane == 0) ? v0 * col[k] : 0.0;
-        for (int r = k + 1 + lane; r < n; r += 32) wv = fma(vk[r], col[r], wv);
-        for (int o = 16; o > 0; o >>= 1) wv += __shfl_xor_sync(0xffffffffu, wv, o);
-        const double bw = beta * wv;
-        if (lane == 0) col[k] = fma(bw, v0, col[k]);
-        for (int r = k + 1 + lane; r < n; r += 32) col[r] = fma(bw, vk[r], col[r]);
-      }
-      __syncthreads();
-      if (tid == 0) vk[k] = g;
-      for (int r = k + 1 + tid; r < n; r += nt) vk[r] = 0.0;
-      __syncthreads();
-    }
-    // a last panel narrower than CS_HB: its unused reflectors are the identity
-    for (int e = tid; e < (CS_HB - kb) * CS_QLD; e += nt) V[kb * CS_QLD + e] = 0.0;
-    for (int e = tid; e < (CS_HB - kb) * CS_HB; e += nt) Tm[kb * CS_HB + e] = 0.0;
-    // ---- T: G = V^T V (upper part), then T column by column
-    for (int e = tid; e < kb * kb; e += nt) {
-      const int i = e / kb, j = e - i * kb;
-      if (j < i) {
-        const double* vi = V + i * CS_QLD;
-        const double* vj = V + j * CS_QLD;
-        double d = 0.0;
-        for (int r = k0 + i; r < n; ++r) d = fma(vj[r], vi[r], d);
-        G[i * CS_HB + j] = d;
-      }
-    }
-    __syncthreads();
-    if (tid == 0) {
-      for (int i = 0; i < kb; ++i) {
-        const double ti = tau[i];
-        for (int j = 0; j < i; ++j) {
-          double sj = 0.0;
-          for (int q = j; q < i; ++q) sj = fma(Tm[q * CS_HB + j], G[i * CS_HB + q], sj);
-          Tm[i * CS_HB + j] = -ti * sj;
-        }
-        Tm[i * CS_HB + i] = ti;
-      }
-    }
-    __syncthreads();
-    // ---- trailing columns: C <- C - V (T^T (V^T C)); four consecutive lanes
-    //      per column, each over every fourth row, V^T C summed across them
-    const int nc = CS_QC - pe;
-    for (int base = 0; base < 4 * nc; base += nt) {
-      const int u = base + tid;
-      const int c = pe + (u >> 2), part = u & 3;
-      const bool act = c < CS_QC;
-      double* col = Q + (size_t)(act ? c : pe) * CS_QLD;
-      double wv[CS_HB];
-#pragma unroll
-      for (int i = 0; i < CS_HB; ++i) wv[i] = 0.0;
-#pragma unroll 2
-      for (int r = k0 + part; r < n; r += 4) {
-        const double x = col[r];
-#pragma unroll
-        for (int i = 0; i < CS_HB; ++i) wv[i] = fma(V[i * CS_QLD + r], x, wv[i]);
-      }
-#pragma unroll
-      for (int i = 0; i < CS_HB; ++i) {
-        wv[i] += __shfl_xor_sync(0xffffffffu, wv[i], 1);
-        wv[i] += __shfl_xor_sync(0xffffffffu, wv[i], 2);
-      }
-      double tw[CS_HB];
-#pragma unroll
-      for (int i = 0; i < CS_HB; ++i) {
-        double sacc = 0.0;
-#pragma unroll
-        for (int j = 0; j <= i; ++j) sacc = fma(Tm[i * CS_HB + j], wv[j], sacc);
-        tw[i] = sacc;
-      }
-      if (act) {
-#pragma unroll 2
-        for (int r = k0 + part; r < n; r += 4) {
-          double x = col[r];
-#pragma unroll
-          for (int i = 0; i < CS_HB; ++i) x = fma(-V[i * CS_QLD + r], tw[i], x);
-          col[r] = x;
-        }
-      }
-    }
-    __syncthreads();
-  }
+  cs_cluster_sync(G);
+  cs_qr_blocked<2 * CS_NY, CS_QLD, CS_TREE_TB>(Q, 2 * CS_NY, CS_QC, CS_NY, level0 ? CS_NY : 0, rank, G, sh, Rd);
   for (int e = tid; e < CS_QC * CS_NY; e += nt) {
     const int c = e / CS_NY, r = e - c * CS_NY;
-    rec[e] = Q[(size_t)c * CS_QLD + r];
+    if (((c >> 3) % G) != rank) continue;
+    const int k0 = c & ~(CS_HQ - 1);
+    double v;
+    if (c >= CS_NY || r < k0) v = Q[(size_t)c * CS_QLD + r];
+    else v = (r <= c) ? Rd[c * CS_HQ + (r - k0)] : 0.0;
+    rec[e] = v;
     if (c >= CS_NY) out_row[(size_t)(c - CS_NY) * CS_NY + r] = Q[(size_t)c * CS_QLD + CS_NY + r];
   }
-  __syncthreads();
+  cs_cluster_sync(G);
 }
 
 #if CS_PREC_TREE != 0
@@ -3618,14 +3805,18 @@ __device__ void cs_merge_cta_lp(const double* ra, const double* rb, double* out_
 }
 #endif  // CS_PREC_TREE != 0
 
-extern "C" __global__ void __launch_bounds__(256) k_tree_level(CsBatch bt, int l) {
+// one merge per CTA, or per cluster of G CTAs
+extern "C" __global__ void __launch_bounds__(CS_TREE_TB, CS_NY <= 256 ? 512 / CS_TREE_TB : 1) k_tree_level(CsBatch bt, int l) {
   extern __shared__ double smem[];
+  const int G = (int)cs_cluster_size(), rank = (int)cs_cluster_rank();
+  const int first = (int)blockIdx.x - rank;  // the cluster's first CTA owns its slab
 #if CS_PREC_TREE == 0
-  if (!cs_big_ok(bt, CS_WS_TREE, CS_SM_TREE)) return;
-  double* Q = CS_Q_SMEM ? smem : bt.wsp + (size_t)blockIdx.x * bt.wsp_stride;
-  double* sh = CS_Q_SMEM ? smem + CS_QSZ : smem;
+  if (!cs_big_ok(bt, CS_WS_TREE, CS_SM_TREE, first + G - 1)) return;
+  double* Q = bt.wsp + (size_t)first * bt.wsp_stride;
+  double* sh = smem;
+  double* Rd = bt.wsp + (size_t)blockIdx.x * bt.wsp_stride + CS_QSZ;
 #else
-  if (!cs_big_ok(bt, CS_WS_TREE_LP, CS_SM_TREE_LP)) return;
+  if (!cs_big_ok(bt, CS_WS_TREE_LP, CS_SM_TREE_LP, blockIdx.x)) return;
   float* Q = reinterpret_cast<float*>(CS_Q_SMEM_LP ? smem : bt.wsp + (size_t)blockIdx.x * bt.wsp_stride);
   double* sh = CS_Q_SMEM_LP ? smem + CS_QSZ_LP : smem;
 #endif
@@ -3634,7 +3825,7 @@ extern "C" __global__ void __launch_bounds__(256) k_tree_level(CsBatch bt, int l
   const long long total = pre[njac];
   const double* srcb = (l & 1) ? bt.rows1 : bt.rows0;
   double* dstb = (l & 1) ? bt.rows0 : bt.rows1;
-  for (long long it = blockIdx.x; it < total; it += gridDim.x) {
+  for (long long it = first / G; it < total; it += gridDim.x / G) {
     const int k = cs_find(pre, njac, it);
     const int b = bt.jac[k];
     const int mi = (int)(it - pre[k]);
@@ -3646,7 +3837,7 @@ extern "C" __global__ void __launch_bounds__(256) k_tree_level(CsBatch bt, int l
     if (mi < merges) {
 #if CS_PREC_TREE == 0
       cs_merge_cta(src + (size_t)(2 * mi) * CS_ROWSZ, src + (size_t)(2 * mi + 1) * CS_ROWSZ, dst + (size_t)mi * CS_ROWSZ,
-                   bt.tree + (size_t)(off + ((2 * mi + 1) << l)) * CS_TREESZ, Q, sh);
+                   bt.tree + (size_t)(off + ((2 * mi + 1) << l)) * CS_TREESZ, Q, sh, Rd, l == 0, rank, G);
 #else
       cs_merge_cta_lp<CS_PREC_TREE>(src + (size_t)(2 * mi) * CS_ROWSZ, src + (size_t)(2 * mi + 1) * CS_ROWSZ,
                                dst + (size_t)mi * CS_ROWSZ, bt.tree + (size_t)(off + ((2 * mi + 1) << l)) * CS_TREESZ, Q,
@@ -3655,30 +3846,36 @@ extern "C" __global__ void __launch_bounds__(256) k_tree_level(CsBatch bt, int l
     } else {
       const double* sr = src + (size_t)(nl - 1) * CS_ROWSZ;
       double* dr = dst + (size_t)merges * CS_ROWSZ;
-      for (int q = threadIdx.x; q < CS_ROWSZ; q += blockDim.x) dr[q] = sr[q];
+      for (int q = threadIdx.x + rank * blockDim.x; q < CS_ROWSZ; q += blockDim.x * G) dr[q] = sr[q];
       __syncthreads();
     }
   }
 }
 
-// Top of the tree, one CTA per instance (as cs_top_warp; Dr goes to the slab).
+// Top of the tree, one CTA or cluster per instance (as cs_top_warp; the system
+// and Dr in the slab).
 // dyk, dpk (refinement, else null): the system is solved for a correction of
 // the direction (dyk, dpk), so the boundary rows' right-hand side is their
 // residual -r - Dr [dy_0; dy_n; dp] (FP64).
 __device__ void cs_top_big(const CsBatch& bt, double* smem, const double* dyk, const double* dpk) {
-  double* slab = bt.wsp + (size_t)blockIdx.x * bt.wsp_stride;
-  double* top = CS_T_SMEM ? smem : slab;
-  double* Dr = CS_T_SMEM ? slab : slab + CS_TSZ;
-  double* red = CS_T_SMEM ? smem + CS_TSZ : smem;
+  const int G = (int)cs_cluster_size(), rank = (int)cs_cluster_rank();
+  const int first = (int)blockIdx.x - rank;
+  if (!cs_big_ok(bt, CS_WS_TOP, CS_SM_TOP, first + G - 1)) return;
+  double* top = bt.wsp + (size_t)first * bt.wsp_stride;
+  double* Dr = top + CS_TSZ;
+  double* Rd = bt.wsp + (size_t)blockIdx.x * bt.wsp_stride + CS_TSZ + CS_DRSZ;
+  double* rhs = Rd + CS_HQ * CS_NT;
+  double* inv = rhs + CS_NT;
+  double* sh = CS_TQ_SMEM ? smem : inv + CS_NT;
   const int tid = threadIdx.x, nt = blockDim.x;
   const int njac = bt.nlist[1];
-  for (int k = blockIdx.x; k < njac; k += gridDim.x) {
+  for (int k = first / G; k < njac; k += gridDim.x / G) {
     const int b = bt.jac[k];
     const int N = bt.N[b], off = bt.off[b];
     const int L = cs_levels(N - 1);
     const double* row = ((L & 1) ? bt.rows1 : bt.rows0) + (size_t)off * CS_ROWSZ;
     const double* th = bt.th + (size_t)b * (CS_NTH > 0 ? CS_NTH : 1);
-    if (tid == 0) {
+    if (tid == 0 && rank == 0) {
       double ya[CS_NY], yb[CS_NY], pl[CS_NP > 0 ? CS_NP : 1];
       for (int q = 0; q < CS_NY; ++q) { ya[q] = bt.y[(size_t)off * CS_NY + q]; yb[q] = bt.y[(size_t)(off + N - 1) * CS_NY + q]; }
       for (int q = 0; q < CS_NP; ++q) pl[q] = bt.p[(size_t)b * CS_NP + q];
@@ -3687,65 +3884,85 @@ __device__ void cs_top_big(const CsBatch& bt, double* smem, const double* dyk, c
       cs_Dr(ya, yb, pl, th, Dr);
       for (int q = 0; q < CS_NY + CS_NP; ++q) top[(size_t)CS_NT * CS_TLD + CS_NY + q] = -r[q];
     }
-    __syncthreads();
+    cs_cluster_sync(G);
     for (int e = tid; e < CS_NT * CS_NT; e += nt) {
       const int c = e / CS_NT, r = e - c * CS_NT;
+      if (((c >> 3) % G) != rank) continue;
       double v;
       if (r < CS_NY) v = (c < 2 * CS_NY + CS_NPE) ? row[c * CS_NY + r] : 0.0;
-      else v = Dr[(r - CS_NY) * (2 * CS_NY + CS_NP) + c];
+      else v = __ldcg(Dr + (size_t)(r - CS_NY) * (2 * CS_NY + CS_NP) + c);
       top[(size_t)c * CS_TLD + r] = v;
     }
-    for (int r = tid; r < CS_NY; r += nt) top[(size_t)CS_NT * CS_TLD + r] = row[(2 * CS_NY + CS_NPE) * CS_NY + r];
-    if (dyk != nullptr) {
-      for (int q = tid; q < CS_NY + CS_NP; q += nt) {
-        const double* dr = Dr + (size_t)q * (2 * CS_NY + CS_NP);
-        double v = top[(size_t)CS_NT * CS_TLD + CS_NY + q];
-        for (int c = 0; c < CS_NY; ++c) v = fma(-dr[c], dyk[(size_t)off * CS_NY + c], v);
-        for (int c = 0; c < CS_NY; ++c) v = fma(-dr[CS_NY + c], dyk[(size_t)(off + N - 1) * CS_NY + c], v);
-        for (int c = 0; c < CS_NP; ++c) v = fma(-dr[2 * CS_NY + c], dpk[(size_t)b * CS_NP + c], v);
-        top[(size_t)CS_NT * CS_TLD + CS_NY + q] = v;
+    if (rank == 0) {
+      for (int r = tid; r < CS_NY; r += nt) top[(size_t)CS_NT * CS_TLD + r] = row[(2 * CS_NY + CS_NPE) * CS_NY + r];
+      if (dyk != nullptr) {
+        for (int q = tid; q < CS_NY + CS_NP; q += nt) {
+          const double* dr = Dr + (size_t)q * (2 * CS_NY + CS_NP);
+          double v = top[(size_t)CS_NT * CS_TLD + CS_NY + q];
+          for (int c = 0; c < CS_NY; ++c) v = fma(-dr[c], dyk[(size_t)off * CS_NY + c], v);
+          for (int c = 0; c < CS_NY; ++c) v = fma(-dr[CS_NY + c], dyk[(size_t)(off + N - 1) * CS_NY + c], v);
+          for (int c = 0; c < CS_NP; ++c) v = fma(-dr[2 * CS_NY + c], dpk[(size_t)b * CS_NP + c], v);
+          top[(size_t)CS_NT * CS_TLD + CS_NY + q] = v;
+        }
       }
     }
-    __syncthreads();
+    cs_cluster_sync(G);
+    cs_qr_blocked<CS_NT, CS_TLD, 256>(top, CS_NT, CS_NT + 1, CS_NT, 0, rank, G, sh, Rd);
+    if (rank == 0) {
+      // back substitution, column-oriented; the next column is on its way
+      // while this one is applied
+      bool zero = false;
+      for (int q = tid; q < CS_NT; q += nt) {
+        const double d = Rd[q * CS_HQ + (q & (CS_HQ - 1))];
+        rhs[q] = __ldcg(top + (size_t)CS_NT * CS_TLD + q);
+        zero |= d == 0.0;
+        inv[q] = d != 0.0 ? cs_rcp(d) : 0.0;
+      }
+      const bool sing = __syncthreads_or(zero) != 0;
+      constexpr int RPT = (CS_NT + 255) / 256;
+      auto entry = [&](int q, int r) -> double {
+        const int k0 = r & ~(CS_HQ - 1);
+        return q < k0 ? __ldcg(top + (size_t)r * CS_TLD + q) : Rd[r * CS_HQ + (q - k0)];
+      };
+      double nx[RPT];
+#pragma unroll
+      for (int s = 0; s < RPT; ++s) nx[s] = (tid + 256 * s < CS_NT - 1) ? entry(tid + 256 * s, CS_NT - 1) : 0.0;
 #pragma unroll 1
-    for (int kk = 0; kk < CS_NT; ++kk) cs_householder_cta(top, CS_TLD, CS_NT, CS_NT + 1, kk, red);
-    // back substitution, column-oriented
-    double* rhs = top + (size_t)CS_NT * CS_TLD;
-    bool sing = false;
-#pragma unroll 1
-    for (int r = CS_NT - 1; r >= 0; --r) {
-      const double d = top[(size_t)r * CS_TLD + r];
-      sing |= (d == 0.0);
-      const double xr = (d != 0.0) ? rhs[r] / d : 0.0;
-      __syncthreads();
-      if (tid == 0) rhs[r] = xr;
-      for (int q = tid; q < r; q += nt) rhs[q] = fma(-top[(size_t)r * CS_TLD + q], xr, rhs[q]);
-      __syncthreads();
-    }
-    if (tid == 0) {
-      if (sing) {
-        for (int r = 0; r < CS_NT; ++r) rhs[r] = 0.0;
-        bt.inst[b].singular += 1;
+      for (int r = CS_NT - 1; r >= 0; --r) {
+        const double xr = rhs[r] * inv[r];
+        double cu[RPT];
+#pragma unroll
+        for (int s = 0; s < RPT; ++s) {
+          cu[s] = nx[s];
+          nx[s] = (tid + 256 * s < r - 1) ? entry(tid + 256 * s, r - 1) : 0.0;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int s = 0; s < RPT; ++s) {
+          const int q = tid + 256 * s;
+          if (q < r) rhs[q] = fma(-cu[s], xr, rhs[q]);
+          if (q == r) rhs[r] = xr;
+        }
+        __syncthreads();
+      }
+      for (int q = tid; q < CS_NY; q += nt) {
+        bt.dy[(size_t)off * CS_NY + q] = sing ? 0.0 : rhs[q];
+        bt.dy[(size_t)(off + N - 1) * CS_NY + q] = sing ? 0.0 : rhs[CS_NY + q];
+      }
+      for (int q = tid; q < CS_NP; q += nt) bt.dp[(size_t)b * CS_NP + q] = sing ? 0.0 : rhs[2 * CS_NY + q];
+      if (tid == 0) {
+        if (sing) bt.inst[b].singular += 1;
+        bt.inst[b].status = ST_LS;
+        bt.inst[b].alpha_ls = 1.0;
+        bt.inst[b].ls_it = 0;
       }
     }
-    __syncthreads();
-    for (int q = tid; q < CS_NY; q += nt) {
-      bt.dy[(size_t)off * CS_NY + q] = rhs[q];
-      bt.dy[(size_t)(off + N - 1) * CS_NY + q] = rhs[CS_NY + q];
-    }
-    for (int q = tid; q < CS_NP; q += nt) bt.dp[(size_t)b * CS_NP + q] = rhs[2 * CS_NY + q];
-    if (tid == 0) {
-      bt.inst[b].status = ST_LS;
-      bt.inst[b].alpha_ls = 1.0;
-      bt.inst[b].ls_it = 0;
-    }
-    __syncthreads();
+    cs_cluster_sync(G);
   }
 }
 
 extern "C" __global__ void __launch_bounds__(256) k_top(CsBatch bt) {
   extern __shared__ double smem[];
-  if (!cs_big_ok(bt, CS_WS_TOP, CS_SM_TOP)) return;
   cs_top_big(bt, smem, nullptr, nullptr);
 }
 
@@ -3792,7 +4009,6 @@ extern "C" __global__ void k_refine_residual(CsBatch bt, const double* __restric
 // the boundary rows of the correction solve (cs_top_big with dyk, dpk)
 extern "C" __global__ void __launch_bounds__(256) k_top_refine(CsBatch bt, const double* dyk, const double* dpk) {
   extern __shared__ double smem[];
-  if (!cs_big_ok(bt, CS_WS_TOP, CS_SM_TOP)) return;
   cs_top_big(bt, smem, dyk, dpk);
 }
 

@@ -57,6 +57,7 @@ struct DriverApi {
   decltype(&cuModuleGetGlobal) moduleGetGlobal = nullptr;
   decltype(&cuModuleUnload) moduleUnload = nullptr;
   decltype(&cuLaunchKernel) launchKernel = nullptr;
+  decltype(&cuLaunchKernelEx) launchKernelEx = nullptr;
   decltype(&cuFuncSetAttribute) funcSetAttribute = nullptr;
   decltype(&cuGetErrorString) getErrorString = nullptr;
   decltype(&cuOccupancyMaxActiveBlocksPerMultiprocessor) occupancy = nullptr;
@@ -210,6 +211,7 @@ int ensure_context() {
     CS_TRY(resolve("cuModuleGetGlobal", (void**)&g_drv.moduleGetGlobal));
     CS_TRY(resolve("cuModuleUnload", (void**)&g_drv.moduleUnload));
     CS_TRY(resolve("cuLaunchKernel", (void**)&g_drv.launchKernel));
+    CS_TRY(resolve("cuLaunchKernelEx", (void**)&g_drv.launchKernelEx));
     CS_TRY(resolve("cuFuncSetAttribute", (void**)&g_drv.funcSetAttribute));
     CS_TRY(resolve("cuGetErrorString", (void**)&g_drv.getErrorString));
     CS_TRY(resolve("cuOccupancyMaxActiveBlocksPerMultiprocessor", (void**)&g_drv.occupancy));
@@ -413,6 +415,7 @@ struct cs_module {
   int condense_block, condense_per_cta;
   size_t condense_smem;
   size_t tree_smem;   // per CTA of 4 warps
+  unsigned tree_block = 256;  // large systems: threads per merge
   int top_wpc;
   size_t top_smem;
   int sms = 1;
@@ -555,7 +558,12 @@ extern "C" int cs_module_load(const cs_module_desc* d, cs_module** out) {
   M->prec = (d->precision == 0) ? 0 : ((d->precision == 1 || d->precision == 3) ? 1 : 2);
   M->prec_tree = (d->precision == 3) ? 1 : ((d->precision == 4) ? 2 : 0);
   M->big_cond = d->layout == 2 || d->precision != 0 || (d->layout == 0 && (!fits_cond || gl > 32));
-  M->big_tree = d->layout == 2 || (d->layout == 0 && !fits_tree);
+  // (from blocks of 28 on a CTA or cluster per merge is faster than a warp per
+  // merge in shared memory whatever the batch: one instance of 1,025 nodes /
+  // 256 of 257, ms for tree, top and back substitution: ny 32 6.9 / 64.1 against
+  // 2.9 / 45.9, ny 28 5.1 / 46.5 against 2.4 / 34.4; at ny 24 3.6 / 22.7
+  // against 1.8 / 23.3 the warp wins where there are many merges)
+  M->big_tree = d->layout == 2 || (d->layout == 0 && (!fits_tree || d->ny >= 28));
   M->big = M->big_cond || M->big_tree;
   M->cgw = gl;
   M->grp_bytes = grp;
@@ -572,11 +580,15 @@ extern "C" int cs_module_load(const cs_module_desc* d, cs_module** out) {
     const long long sm_cond = (long long)s1 * (nb + 1) + nb * ldg + (long long)d->m * rb + d->m * d->m + d->ny + s1 + 16 + nb;
     const long long qsz = (long long)qld * qc, tsz = (long long)tld * (nt + 1);
     const long long drsz = (long long)(d->ny + d->np) * (2 * d->ny + d->np);
-    const long long hb = 16, sm_hb = hb * qld + 2 * hb * hb + hb + 32;
-    const bool q_smem = (qsz + sm_hb) * 8 <= smem_optin, t_smem = (tsz + 32) * 8 <= smem_optin;
+    // CS_SM_QR(ld) in cs_kernels.cuh
+    const long long hb = 16, hq = 8;
+    auto sm_qr = [&](long long ld) { return hq * ld + hq * hq + 12 * hq; };
+    const long long sm_hb = sm_qr(qld);
+    const bool tq_smem = sm_qr(tld) * 8 <= smem_optin;
+    const long long sm_top = tq_smem ? sm_qr(tld) : 0;
     M->slab = 0;
     if (M->big_cond) M->slab = std::max(M->slab, ws_cond);
-    if (M->big_tree) M->slab = std::max(M->slab, std::max(q_smem ? 0ll : qsz, (t_smem ? 0ll : tsz) + drsz));
+    if (M->big_tree) M->slab = std::max(M->slab, std::max(qsz + hq * d->ny, tsz + drsz + (hq + 2) * nt + (tq_smem ? 0 : sm_qr(tld))));
     if (M->big_cond) {
       M->condense_smem = (size_t)sm_cond * 8;
       if (M->prec) {
@@ -612,14 +624,14 @@ extern "C" int cs_module_load(const cs_module_desc* d, cs_module** out) {
       const long long shf = hb * qld + 2 * hb * hb + hb + (long long)qc * hb, sm_hb_lp = (shf + 1) / 2 + 32;
       const long long qsz_lp = (qsz + 1) / 2;
       const bool q_smem_lp = (qsz_lp + sm_hb_lp) * 8 <= smem_optin;
-      M->slab = std::max(M->slab, std::max(q_smem_lp ? 0ll : qsz_lp, (t_smem ? 0ll : tsz) + drsz));
       M->tree_smem = (size_t)((q_smem_lp ? qsz_lp : 0) + sm_hb_lp) * 8;
-      M->top_smem = (size_t)((t_smem ? tsz : 0) + 32) * 8;
+      M->top_smem = (size_t)sm_top * 8;
       M->top_wpc = 8;
       M->babd_cta_smem = 0;
     } else if (M->big_tree) {
-      M->tree_smem = (size_t)((q_smem ? qsz : 0) + sm_hb) * 8;
-      M->top_smem = (size_t)((t_smem ? tsz : 0) + 32) * 8;
+      M->tree_smem = (size_t)sm_hb * 8;
+      M->tree_block = d->ny <= 32 ? 64 : (d->ny <= 64 ? 128 : 256);  // CS_TREE_TB
+      M->top_smem = (size_t)sm_top * 8;
       M->top_wpc = 8;
       M->babd_cta_smem = 0;
     }
@@ -762,9 +774,9 @@ extern "C" int cs_module_load(const cs_module_desc* d, cs_module** out) {
     }
     if (M->big_tree) {
       int pt = 0;
-      CS_CU(g_drv.occupancy(&pt, M->f_tree_level, 256, M->tree_smem));
+      CS_CU(g_drv.occupancy(&pt, M->f_tree_level, (int)M->tree_block, M->tree_smem));
       M->tree_grid = M->sms * std::max(1, pt);
-      M->big_ctas = std::max(M->big_ctas, M->tree_grid);
+      M->big_ctas = std::max(M->big_ctas, std::max(M->tree_grid, M->sms));
     }
   }
   {
@@ -1043,29 +1055,64 @@ static int flush_events(cs_batch* bt) {
   return CS_OK;
 }
 
-// kind: -1 untimed, 0 condense, 1 babd, 2 residual
-static int launch_k(cs_batch* bt, CUfunction f, unsigned grid, unsigned block, size_t smem, void** args, int kind) {
-  if (grid == 0) return CS_OK;
-  cs_batch::EvPair* ev = nullptr;
-  if (bt->timing && kind >= 0) {
+// events around a launch of a timed kind (-1 untimed, 0 condense, 1 babd, 2
+// residual)
+static int event_begin(cs_batch* bt, int kind, cs_batch::EvPair** out) {
+  *out = nullptr;
+  if (!bt->timing || kind < 0) return CS_OK;
+  if (bt->ev_used == bt->ev_pool.size()) {
+    if (bt->ev_pool.size() >= 3072) CS_TRY(flush_events(bt));
     if (bt->ev_used == bt->ev_pool.size()) {
-      if (bt->ev_pool.size() >= 3072) CS_TRY(flush_events(bt));
-      if (bt->ev_used == bt->ev_pool.size()) {
-        cs_batch::EvPair e;
-        CS_CUDA(cudaEventCreate(&e.a));
-        CS_CUDA(cudaEventCreate(&e.b));
-        bt->ev_pool.push_back(e);
-      }
+      cs_batch::EvPair e;
+      CS_CUDA(cudaEventCreate(&e.a));
+      CS_CUDA(cudaEventCreate(&e.b));
+      bt->ev_pool.push_back(e);
     }
-    ev = &bt->ev_pool[bt->ev_used++];
-    ev->kind = kind;
-    CS_CUDA(cudaEventRecord(ev->a, bt->stream));
   }
-  CS_CU(g_drv.launchKernel(f, grid, 1, 1, block, 1, 1, (unsigned)smem, (CUstream)bt->stream, args, nullptr));
+  *out = &bt->ev_pool[bt->ev_used++];
+  (*out)->kind = kind;
+  CS_CUDA(cudaEventRecord((*out)->a, bt->stream));
+  return CS_OK;
+}
+static int event_end(cs_batch* bt, int kind, cs_batch::EvPair* ev) {
   bt->launches += 1;
   if (kind >= 0) bt->kind_launches[kind] += 1;
   if (ev) CS_CUDA(cudaEventRecord(ev->b, bt->stream));
   return CS_OK;
+}
+
+static int launch_k(cs_batch* bt, CUfunction f, unsigned grid, unsigned block, size_t smem, void** args, int kind) {
+  if (grid == 0) return CS_OK;
+  cs_batch::EvPair* ev = nullptr;
+  CS_TRY(event_begin(bt, kind, &ev));
+  CS_CU(g_drv.launchKernel(f, grid, 1, 1, block, 1, 1, (unsigned)smem, (CUstream)bt->stream, args, nullptr));
+  return event_end(bt, kind, ev);
+}
+
+// the same with clusters of `cluster` CTAs (grid a multiple of it), untimed kinds
+// as launch_k's
+static int launch_cluster(cs_batch* bt, CUfunction f, unsigned grid, unsigned block, size_t smem, unsigned cluster,
+                          void** args, int kind) {
+  if (cluster <= 1 || grid == 0) return launch_k(bt, f, grid, block, smem, args, kind);
+  CUlaunchAttribute at;
+  memset(&at, 0, sizeof(at));
+  at.id = CU_LAUNCH_ATTRIBUTE_CLUSTER_DIMENSION;
+  at.value.clusterDim.x = cluster;
+  at.value.clusterDim.y = at.value.clusterDim.z = 1;
+  CUlaunchConfig cfg;
+  memset(&cfg, 0, sizeof(cfg));
+  cfg.gridDimX = grid;
+  cfg.gridDimY = cfg.gridDimZ = 1;
+  cfg.blockDimX = block;
+  cfg.blockDimY = cfg.blockDimZ = 1;
+  cfg.sharedMemBytes = (unsigned)smem;
+  cfg.hStream = (CUstream)bt->stream;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  cs_batch::EvPair* ev = nullptr;
+  CS_TRY(event_begin(bt, kind, &ev));
+  CS_CU(g_drv.launchKernelEx(&cfg, f, args, nullptr));
+  return event_end(bt, kind, ev);
 }
 
 static int launch(cs_batch* bt, CUfunction f, unsigned grid, unsigned block, size_t smem, void** args) {
@@ -1165,6 +1212,35 @@ static int run_lists(cs_batch* bt, CsBatchDev& v, int mode, int nlvl, const CsCo
 // work lists
 static const int kDecideInLists = 4096;
 
+// CTAs per merge (or top system) of a large-system launch with `work` of them:
+// the largest cluster up to 8 that still gives each CTA an SM of its own.  (One
+// CTA alone is bound by its SM's FP64 unit; two CTAs on one SM would share it.)
+static unsigned cluster_for(const cs_module* M, long long work) {
+  unsigned g = 1;
+  while (g < 8 && work * 2 * g <= M->sms) g *= 2;
+  return g;
+}
+
+// large systems: tree level l, a cluster of CTAs per merge where the level has
+// fewer merges than the GPU has SMs
+static int run_big_level(cs_batch* bt, int l, void** args, unsigned gtree) {
+  cs_module* M = bt->M;
+  long long items = 0;
+  for (int n : bt->hN) {
+    int r = n - 1;
+    for (int q = 0; q < l; ++q) r = (r + 1) >> 1;
+    if (r > 1) items += (r + 1) >> 1;
+  }
+  // in the tail at most the capped slots' worth
+  if (bt->work_cap > 0) items = std::min<long long>(items, (bt->work_cap >> (l + 1)) + bt->inst_cap);
+  const unsigned cl = M->prec_tree ? 1 : cluster_for(M, std::max<long long>(items, 1));
+  // (one merge per SM: with room for more, two of 128 merges shared an SM)
+  if (cl == 1 && items <= M->sms) gtree = std::min(gtree, (unsigned)M->sms);
+  if (cl == 1) return launch_k(bt, M->f_tree_level, gtree, M->tree_block, M->tree_smem, args, 1);
+  return launch_cluster(bt, M->f_tree_level, (unsigned)std::max<long long>(items, 1) * cl, M->tree_block, M->tree_smem, cl,
+                        args, 1);
+}
+
 // Newton direction for the instances on the jac list: tree levels up, top
 // system, back substitution down, stage recovery.
 static int run_direction(cs_batch* bt, CsBatchDev& v, int nlvl) {
@@ -1186,10 +1262,12 @@ static int run_direction(cs_batch* bt, CsBatchDev& v, int nlvl) {
   // merges of a level <= slots; per CTA: one (large), at least 4 (warps / lanes)
   const unsigned gtree = M->big_tree ? capped(bt, (unsigned)M->tree_grid, 1, 1)
                                      : capped(bt, (unsigned)M->tree_small_grid, 1, 4);
-  const unsigned gback = capped(bt, g, 1, 4);
+  // top system of a large-system tree: a cluster per instance
+  const unsigned inst = capped_inst(bt, (unsigned)bt->B), ctop = cluster_for(M, inst);
+  const unsigned gtop = M->big_tree ? std::min(inst, (unsigned)M->big_ctas / ctop) * ctop : 0;
   for (int l = 0; l < l_lo; ++l) {
     void* a[] = {&v, &l};
-    if (M->big_tree) CS_TRY(launch_k(bt, M->f_tree_level, gtree, 256, M->tree_smem, a, 1));
+    if (M->big_tree) CS_TRY(run_big_level(bt, l, a, gtree));
     else CS_TRY(launch_k(bt, M->f_tree_level, gtree, 128, M->tree_smem, a, 1));
   }
   if (M->upper && bt->opts.babd_path != 2) {
@@ -1198,13 +1276,15 @@ static int run_direction(cs_batch* bt, CsBatchDev& v, int nlvl) {
     CS_TRY(launch_k(bt, M->f_upper, capped_inst(bt, (unsigned)std::min(M->upper_grid, bt->B)), 128, 0, a, 1));
   } else {
     void* a[] = {&v};
-    if (M->big_tree)
-      CS_TRY(launch_k(bt, M->f_top, capped_inst(bt, (unsigned)std::min(M->big_ctas, bt->B)), 256, M->top_smem, a, 1));
+    if (M->big_tree) CS_TRY(launch_cluster(bt, M->f_top, gtop, 256, M->top_smem, ctop, a, 1));
     else CS_TRY(launch_k(bt, M->f_top, capped_inst(bt, (unsigned)(M->sms * 4)), 32 * M->top_wpc, M->top_smem, a, 1));
   }
+  // (large blocks: a CTA of 256 threads per merge)
+  const unsigned bback = M->big_tree ? 256 : 128;
+  const unsigned gback = M->big_tree ? capped(bt, g, 1, 1) : capped(bt, g, 1, 4);
   for (int l = l_lo - 1; l >= 0; --l) {
     void* a[] = {&v, &l};
-    CS_TRY(launch_k(bt, M->f_backsub_level, gback, 128, 0, a, 1));
+    CS_TRY(launch_k(bt, M->f_backsub_level, gback, bback, 0, a, 1));
   }
   if (refine) {
     // FP64 iterative refinement: residual of the condensed system at the
@@ -1220,11 +1300,10 @@ static int run_direction(cs_batch* bt, CsBatchDev& v, int nlvl) {
         CS_TRY(launch_k(bt, M->f_tree_level, gtree, 256, M->tree_smem, a, 1));
       }
       void* at[] = {&v, &dyk, &dpk};
-      CS_TRY(launch_k(bt, M->f_top_refine, capped_inst(bt, (unsigned)std::min(M->big_ctas, bt->B)), 256,
-                      M->top_smem, at, 1));
+      CS_TRY(launch_cluster(bt, M->f_top_refine, gtop, 256, M->top_smem, ctop, at, 1));
       for (int l = l_lo - 1; l >= 0; --l) {
         void* a[] = {&v, &l};
-        CS_TRY(launch_k(bt, M->f_backsub_level, gback, 128, 0, a, 1));
+        CS_TRY(launch_k(bt, M->f_backsub_level, gback, bback, 0, a, 1));
       }
       CS_TRY(launch_k(bt, M->f_refine_add, capped(bt, g, 1, 4), 128, 0, at, 1));
     }
