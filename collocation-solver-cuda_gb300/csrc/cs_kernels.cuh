@@ -2452,8 +2452,13 @@ extern "C" __global__ void k_babd_cta(CsBatch bt) {}
 //       | (reduced precision) FP32 copies of the stage Jacobians and X0
 #define CS_WS_JF ((long long)CS_M * CS_RB * CS_NFG + (long long)CS_RB * CS_NRHS + CS_M * CS_M + CS_M)
 #define CS_WS_COND ((long long)CS_S1 * CS_LDG + CS_WS_JF + (CS_PREC ? (CS_WS_JF + 1) / 2 : 0ll))
-// shared: panel [S1][PLD] | U12 [NB][LDG] | fa [M RB] | hA [M M] | fb [NY] | inv [S1] | red [16] | piv [NB]
-#define CS_SM_COND (CS_S1 * CS_PLD + CS_NB * CS_LDG + CS_M * CS_RB + CS_M * CS_M + CS_NY + CS_S1 + 16 + CS_NB)
+// shared: panel [S1][PLD] | U12 [NB][LDG] | fa [M RB] | hA [M M] | fb [NY] | inv [S1] | red [16] |
+//         rows kk and pivot [2][NB] | swapped rows, source and destination [4 NB ints]
+#define CS_SM_COND (CS_S1 * CS_PLD + CS_NB * CS_LDG + CS_M * CS_RB + CS_M * CS_M + CS_NY + CS_S1 + 16 + 4 * CS_NB)
+// threads, and the columns of the first panel: what is left over by the others,
+// so that the rows below every panel fill the 16-row tiles of the update
+#define CS_COND_TB (CS_S1 <= 128 ? 128 : 256)
+#define CS_KB0 (CS_S1 % CS_NB ? CS_S1 % CS_NB : CS_NB)
 // merge matrix and top system: in shared memory when they fit, else in the slab
 #define CS_QSZ (CS_QLD * CS_QC)
 #define CS_TSZ (CS_TLD * (CS_NT + 1))
@@ -2512,6 +2517,14 @@ __device__ __forceinline__ bool cs_big_ok(const CsBatch& bt, long long slab, lon
                   (slab == 0 || (bt.wsp != nullptr && last < bt.wsp_ctas && bt.wsp_stride >= slab));
   if (!ok && threadIdx.x == 0) atomicAdd(&bt.counters[7], 1ull);
   return ok;
+}
+
+// largest key over the warp, the smallest row on ties; every lane gets it
+__device__ __forceinline__ void cs_warp_argmax(unsigned long long& best, int& brow) {
+  const unsigned hi = (unsigned)(best >> 32), mh = __reduce_max_sync(0xffffffffu, hi);
+  const unsigned lo = hi == mh ? (unsigned)best : 0u, ml = __reduce_max_sync(0xffffffffu, lo);
+  brow = (int)__reduce_min_sync(0xffffffffu, (hi == mh && (unsigned)best == ml) ? (unsigned)brow : 0x7fffffffu);
+  best = ((unsigned long long)mh << 32) | ml;
 }
 
 // largest key over the CTA, the smallest row on ties (red: 16 doubles)
@@ -2591,7 +2604,8 @@ __device__ void cs_condense_big(const CsBatch& bt, int slot, double* slab, doubl
   double* fb = hA + CS_M * CS_M;
   T* inv = reinterpret_cast<T*>(fb + CS_NY);
   double* red = fb + CS_NY + CS_S1;
-  int* piv = (int*)(red + 16);
+  T* rowx = reinterpret_cast<T*>(red + 16);  // [2][NB]
+  int* moved = (int*)(red + 16 + 2 * CS_NB);  // [64]
   const int b = bt.inst_of[slot];
   const double h = bt.t[slot + 1] - bt.t[slot];
   const double* yi = bt.y + (size_t)slot * CS_NY;
@@ -2668,106 +2682,165 @@ __device__ void cs_condense_big(const CsBatch& bt, int slot, double* slab, doubl
     W[(size_t)row * CS_LDG + col] = (T)v;
   }
   __syncthreads();
-  // ---- blocked LU with partial pivoting
+  // ---- blocked LU with partial pivoting.  Panel: a row per thread in
+  // registers; per column the largest entry by warp maxima of the key's words,
+  // rows kk and pivot exchanged through shared memory, two barriers (six
+  // before).  The row swaps of a panel reach the other columns as one
+  // permutation, all loads before the stores, and U12 is solved in registers: a
+  // swap after the other through the slab and sums through shared memory were a
+  // chain of some 20,000 cycles a panel.  What bounds it is the SM's FP64 unit;
+  // per direction, K = 16 chain (s1 272) 55.4 -> 50.1 ms, K = 8 batch (s1 102)
+  // 18.0 -> 15.7; the same operations on every entry in the same order.
   int singular = 0;
+  const int lane = tid & 31, w = tid >> 5;
+  constexpr int NT = CS_COND_TB, NW = NT / 32, RPT = (CS_S1 + NT - 1) / NT;
 #pragma unroll 1
-  for (int k0 = 0; k0 < CS_S1; k0 += CS_NB) {
-    const int kb = min(CS_NB, CS_S1 - k0);
+  for (int k0 = 0, kb = CS_KB0; k0 < CS_S1; k0 += kb, kb = CS_NB) {
     const int pr = CS_S1 - k0;        // panel rows
-    for (int e = tid; e < pr * kb; e += nt) {
+    for (int e = tid; e < pr * kb; e += NT) {
       const int r = e / kb, c = e - r * kb;
       P[r * CS_PLD + c] = W[(size_t)(k0 + r) * CS_LDG + k0 + c];
     }
     __syncthreads();
-#pragma unroll 1
-    for (int kk = 0; kk < kb; ++kk) {
-      unsigned long long best = 0ull;
-      int brow = CS_S1;  // larger than any row: loses every tie
-      for (int r = kk + tid; r < pr; r += nt) {
-        const unsigned long long v = cs_abskey(P[r * CS_PLD + kk]);
-        if (v > best || brow == CS_S1) { best = v; brow = r; }
-      }
-      cs_cta_argmax(best, brow, red);
-      if (tid == 0) piv[kk] = brow;
-      if (brow != kk)
-        for (int c = tid; c < kb; c += nt) {
-          const T tmp = P[kk * CS_PLD + c];
-          P[kk * CS_PLD + c] = P[brow * CS_PLD + c];
-          P[brow * CS_PLD + c] = tmp;
-        }
-      __syncthreads();
-      const T pv = P[kk * CS_PLD + kk];
-      const bool tiny = cs_tiny(pv);  // |pv| < 10 * 2^-52
-      singular |= tiny;
-      const T ip = (T)1 / pv;
-      if (tid == 0) inv[k0 + kk] = ip;
-      const T mul = tiny ? (T)0 : ip;
-      for (int r = kk + 1 + tid; r < pr; r += nt) P[r * CS_PLD + kk] *= mul;
-      __syncthreads();
-      const int nc = kb - kk - 1;
-      if (nc > 0) {
-        const int ne = (pr - kk - 1) * nc;
-        for (int e = tid; e < ne; e += nt) {
-          const int rr = e / nc;
-          const int r = kk + 1 + rr, c = kk + 1 + (e - rr * nc);
-          P[r * CS_PLD + c] = cs_fma(-P[r * CS_PLD + kk], P[kk * CS_PLD + c], P[r * CS_PLD + c]);
-        }
-      }
-      __syncthreads();
+    T x[RPT][CS_NB];
+#pragma unroll
+    for (int s = 0; s < RPT; ++s) {
+      const int r = tid + NT * s;
+#pragma unroll
+      for (int c = 0; c < CS_NB; ++c) x[s][c] = (r < pr && c < kb) ? P[r * CS_PLD + c] : (T)0;
     }
+    // (warp 0) the rows that the swaps move: lane e < kb row e, lane 16 + i the
+    // i-th row from below the panel's first kb; src: the row that ends there
+    int dst = lane < kb ? lane : -1, src = dst, nmoved = 0;
+    cs_static_for<0, CS_NB>([&](auto kc) {
+      constexpr int kk = decltype(kc)::value;
+      if (kk < kb) {
+        unsigned long long best = 0ull;
+        int brow = CS_S1;  // larger than any row: loses every tie
+#pragma unroll
+        for (int s = 0; s < RPT; ++s) {
+          const int r = tid + NT * s;
+          const unsigned long long v = cs_abskey(x[s][kk]);
+          if (r >= kk && r < pr && (v > best || brow == CS_S1)) { best = v; brow = r; }
+        }
+        cs_warp_argmax(best, brow);
+        if (lane == 0) {
+          red[w] = __longlong_as_double((long long)best);
+          red[8 + w] = (double)brow;
+        }
+        __syncthreads();
+        best = lane < NW ? (unsigned long long)__double_as_longlong(red[lane]) : 0ull;
+        brow = lane < NW ? (int)red[8 + lane] : CS_S1;
+        cs_warp_argmax(best, brow);
+#pragma unroll
+        for (int s = 0; s < RPT; ++s) {
+          const int r = tid + NT * s;
+          if (r == kk) {
+#pragma unroll
+            for (int c = 0; c < CS_NB; ++c) rowx[c] = x[s][c];
+          }
+          if (r == brow) {
+#pragma unroll
+            for (int c = 0; c < CS_NB; ++c) rowx[CS_NB + c] = x[s][c];
+            inv[k0 + kk] = (T)1 / x[s][kk];
+          }
+        }
+        if (w == 0 && brow != kk) {
+          const unsigned m = __ballot_sync(0xffffffffu, dst == brow);
+          const int at = m ? __ffs(m) - 1 : CS_NB + nmoved;
+          if (m == 0) {
+            if (lane == at) dst = src = brow;
+            ++nmoved;
+          }
+          const int s0 = __shfl_sync(0xffffffffu, src, kk), s1 = __shfl_sync(0xffffffffu, src, at);
+          if (lane == kk) src = s1;
+          if (lane == at) src = s0;
+        }
+        __syncthreads();
+        const T pv = rowx[CS_NB + kk];
+        const bool tiny = cs_tiny(pv);  // |pv| < 10 * 2^-52
+        singular |= tiny;
+        const T mul = tiny ? (T)0 : inv[k0 + kk];
+#pragma unroll
+        for (int s = 0; s < RPT; ++s) {
+          const int r = tid + NT * s;
+          if (r == kk || r == brow) {
+            const T* from = rowx + (r == kk ? CS_NB : 0);
+#pragma unroll
+            for (int c = 0; c < CS_NB; ++c) x[s][c] = from[c];
+          }
+          if (r > kk && r < pr) {
+            x[s][kk] *= mul;
+#pragma unroll
+            for (int c = kk + 1; c < CS_NB; ++c) x[s][c] = cs_fma(-x[s][kk], rowx[CS_NB + c], x[s][c]);
+          }
+        }
+      }
+    });
+#pragma unroll
+    for (int s = 0; s < RPT; ++s) {
+      const int r = tid + NT * s;
+#pragma unroll
+      for (int c = 0; c < CS_NB; ++c)
+        if (r < pr && c < kb) P[r * CS_PLD + c] = x[s][c];
+    }
+    if (w == 0) {
+      moved[lane] = src;
+      moved[32 + lane] = dst;
+    }
+    __syncthreads();
     // panel rows 0..kb-1 (U11, multipliers below its diagonal) back to the slab
-    for (int e = tid; e < kb * kb; e += nt) {
+    for (int e = tid; e < kb * kb; e += NT) {
       const int r = e / kb, c = e - r * kb;
       W[(size_t)(k0 + r) * CS_LDG + k0 + c] = P[r * CS_PLD + c];
     }
-    // columns right of the panel: the row swaps in order, then U12 = L11^-1 A12
+    // columns right of the panel: the swapped rows, then U12 = L11^-1 A12
     const int c0 = k0 + kb, ncol = CS_NCOL1 - c0;
-    for (int c = tid; c < ncol; c += nt) {
-      T* colp = W + c0 + c;
-      for (int kk = 0; kk < kb; ++kk) {
-        const int pr2 = piv[kk];
-        if (pr2 != kk) {
-          const T t0 = colp[(size_t)(k0 + kk) * CS_LDG];
-          colp[(size_t)(k0 + kk) * CS_LDG] = colp[(size_t)(k0 + pr2) * CS_LDG];
-          colp[(size_t)(k0 + pr2) * CS_LDG] = t0;
-        }
+    for (int c = tid; c < ncol; c += NT) {
+      T* colp = W + (size_t)k0 * CS_LDG + c0 + c;
+      T v[CS_NB], o[CS_NB];
+#pragma unroll
+      for (int i = 0; i < CS_NB; ++i) {
+        v[i] = i < kb ? colp[(size_t)moved[i] * CS_LDG] : (T)0;
+        o[i] = moved[48 + i] >= 0 ? colp[(size_t)moved[16 + i] * CS_LDG] : (T)0;
       }
-      // column c of U12 in shared memory (this thread's own column)
-#pragma unroll 1
-      for (int i = 0; i < kb; ++i) {
-        T v = colp[(size_t)(k0 + i) * CS_LDG];
-        for (int l = 0; l < i; ++l) v = cs_fma(-P[i * CS_PLD + l], U[l * CS_LDG + c], v);
-        colp[(size_t)(k0 + i) * CS_LDG] = v;
-        U[i * CS_LDG + c] = v;
+#pragma unroll
+      for (int i = 0; i < CS_NB; ++i)
+        if (moved[48 + i] >= 0) colp[(size_t)moved[48 + i] * CS_LDG] = o[i];
+#pragma unroll
+      for (int l = 0; l < CS_NB; ++l) {
+        if (l < kb) {
+          colp[(size_t)l * CS_LDG] = v[l];
+          U[l * CS_LDG + c] = v[l];
+#pragma unroll
+          for (int i = l + 1; i < CS_NB; ++i)
+            if (i < kb) v[i] = cs_fma(-P[i * CS_PLD + l], v[l], v[i]);
+        }
       }
     }
     __syncthreads();
-    // trailing update A22 -= L21 U12: warp items of 16 rows x 32 columns,
-    // lane owns one column (fills the lanes for any trailing width)
+    // trailing update A22 -= L21 U12: 16 rows x 1 column per lane, the columns
+    // of all row tiles in one sequence (no idle lanes at a tile's right edge)
     const int r0 = k0 + kb, nr = CS_S1 - r0;
-    if (nr > 0 && ncol > 0) {
-      const int rt = (nr + 15) >> 4, ct = (ncol + 31) >> 5;
-      const int lane = tid & 31, w = tid >> 5, nw = nt >> 5;
-      for (int item = w; item < rt * ct; item += nw) {
-        const int ri = item / ct, ci = item - ri * ct;
-        const int ra = ri * 16, c = ci * 32 + lane;
-        const bool cok = c < ncol;
-        double acc[16];
+    const int items = (nr >> 4) * ncol;
+    for (int e0 = w * 32; e0 < items; e0 += NT) {
+      const int e = e0 + lane;
+      const bool ok = e < items;
+      const int ri = ok ? e / ncol : 0, c = ok ? e - ri * ncol : 0;
+      T* wp = W + (size_t)(r0 + ri * 16) * CS_LDG + c0 + c;
+      const T* lp = P + (kb + ri * 16) * CS_PLD;
+      double acc[16];
 #pragma unroll
-        for (int i = 0; i < 16; ++i)
-          acc[i] = (cok && ra + i < nr) ? W[(size_t)(r0 + ra + i) * CS_LDG + c0 + c] : 0.0;
+      for (int i = 0; i < 16; ++i) acc[i] = ok ? wp[(size_t)i * CS_LDG] : 0.0;
 #pragma unroll 2
-        for (int l = 0; l < kb; ++l) {
-          const double uv = cok ? U[l * CS_LDG + c] : 0.0;
+      for (int l = 0; l < kb; ++l) {
+        const double uv = U[l * CS_LDG + c];
 #pragma unroll
-          for (int i = 0; i < 16; ++i) {
-            const double lv = (ra + i < nr) ? P[(kb + ra + i) * CS_PLD + l] : 0.0;
-            acc[i] = fma(-lv, uv, acc[i]);
-          }
-        }
+        for (int i = 0; i < 16; ++i) acc[i] = fma(-lp[i * CS_PLD + l], uv, acc[i]);
+      }
+      if (ok) {
 #pragma unroll
-        for (int i = 0; i < 16; ++i)
-          if (cok && ra + i < nr) W[(size_t)(r0 + ra + i) * CS_LDG + c0 + c] = acc[i];
+        for (int i = 0; i < 16; ++i) wp[(size_t)i * CS_LDG] = acc[i];
       }
     }
     __syncthreads();
@@ -2775,8 +2848,9 @@ __device__ void cs_condense_big(const CsBatch& bt, int slot, double* slab, doubl
   // ---- back substitution, blocks of CS_NB rows from the bottom; the
   //      right-hand sides are columns S1.. of the slab rows
 #pragma unroll 1
-  for (int k0 = ((CS_S1 - 1) / CS_NB) * CS_NB; k0 >= 0; k0 -= CS_NB) {
-    const int kb = min(CS_NB, CS_S1 - k0);
+  for (int ke = CS_S1; ke > 0;) {  // the panels' blocks, from the last
+    const int kb = ke > CS_KB0 ? CS_NB : CS_KB0, k0 = ke - kb;
+    ke = k0;
     // U column block [0, k0+kb) x [k0, k0+kb) into the panel buffer
     for (int e = tid; e < (k0 + kb) * kb; e += nt) {
       const int r = e / kb, c = e - r * kb;
@@ -2785,15 +2859,20 @@ __device__ void cs_condense_big(const CsBatch& bt, int slot, double* slab, doubl
     __syncthreads();
     // diagonal block, one thread per right-hand side, rows from the bottom
     for (int c = tid; c < CS_NRHS; c += nt) {
-      T* colp = W + CS_S1 + c;
-      for (int i = 0; i < kb; ++i) U[i * CS_LDG + c] = colp[(size_t)(k0 + i) * CS_LDG];
-#pragma unroll 1
-      for (int i = kb - 1; i >= 0; --i) {
-        const T xi = U[i * CS_LDG + c] * inv[k0 + i];
-        U[i * CS_LDG + c] = xi;
-        for (int q = 0; q < i; ++q) U[q * CS_LDG + c] = cs_fma(-P[(k0 + q) * CS_PLD + i], xi, U[q * CS_LDG + c]);
+      T* colp = W + (size_t)k0 * CS_LDG + CS_S1 + c;
+      T v[CS_NB];
+#pragma unroll
+      for (int i = 0; i < CS_NB; ++i) v[i] = i < kb ? colp[(size_t)i * CS_LDG] : (T)0;
+#pragma unroll
+      for (int i = CS_NB - 1; i >= 0; --i) {
+        if (i < kb) {
+          v[i] *= inv[k0 + i];
+          colp[(size_t)i * CS_LDG] = v[i];
+          U[i * CS_LDG + c] = v[i];
+#pragma unroll
+          for (int q = 0; q < i; ++q) v[q] = cs_fma(-P[(k0 + q) * CS_PLD + i], v[i], v[q]);
+        }
       }
-      for (int i = 0; i < kb; ++i) colp[(size_t)(k0 + i) * CS_LDG] = U[i * CS_LDG + c];
     }
     __syncthreads();
     // rows above the block: B[q] -= U[q][k0 + i] x[i], i from the last
