@@ -448,6 +448,8 @@ def _roofline(groups, fp64_peak):
                            "from MEASURED_PEAKS.json",
             "flops_per_launch": flops / len(groups), "ms_per_launch": cms / len(groups),
             "flops_note": "contract flops per interval (2/3)s^3 + 2 s^2 r, s = m(ny+nz), r = ny+np_eff+1; "
+                          "the kernel executes about half of them (stage 0 and the algebraic unknowns are "
+                          "eliminated apart), so frac can exceed 1; "
                           "algorithmic bytes 8(2 + 2ny + m(ny+nz) + r s + ny(2ny+np_eff+1)) per interval",
             "hbm_gbs": cbytes / (cms * 1e-3) / 1e9}
 

@@ -2464,8 +2464,9 @@ extern "C" __global__ void k_babd_cta(CsBatch bt) {}
 #define CS_WS_JF ((long long)CS_M * CS_RB * CS_NFG + (long long)CS_RB * CS_NRHS + CS_M * CS_M + CS_M)
 #define CS_WS_COND ((long long)CS_S1 * CS_LDG + CS_WS_JF + (CS_PREC ? (CS_WS_JF + 1) / 2 : 0ll))
 // shared: panel [S1][PLD] | U12 [NB][LDG] | fa [M RB] | hA [M M] | fb [NY] | inv [S1] | red [16] |
-//         rows kk and pivot [2][NB] | swapped rows, source and destination [4 NB ints]
-#define CS_SM_COND (CS_S1 * CS_PLD + CS_NB * CS_LDG + CS_M * CS_RB + CS_M * CS_M + CS_NY + CS_S1 + 16 + 4 * CS_NB)
+//         swapped rows, source and destination [4 NB shorts]; rows kk and pivot of
+//         a panel [2][NB] in U12, which is written after it
+#define CS_SM_COND (CS_S1 * CS_PLD + CS_NB * CS_LDG + CS_M * CS_RB + CS_M * CS_M + CS_NY + CS_S1 + 16 + CS_NB)
 // threads, and the columns of the first panel: what is left over by the others,
 // so that the rows below every panel fill the 16-row tiles of the update
 #define CS_COND_TB (CS_S1 <= 128 ? 128 : 256)
@@ -2615,8 +2616,8 @@ __device__ void cs_condense_big(const CsBatch& bt, int slot, double* slab, doubl
   double* fb = hA + CS_M * CS_M;
   T* inv = reinterpret_cast<T*>(fb + CS_NY);
   double* red = fb + CS_NY + CS_S1;
-  T* rowx = reinterpret_cast<T*>(red + 16);  // [2][NB]
-  int* moved = (int*)(red + 16 + 2 * CS_NB);  // [64]
+  T* rowx = U;                        // [2][NB], while U12 is not in use
+  short* moved = (short*)(red + 16);  // [2][2 NB]
   const int b = bt.inst_of[slot];
   const double h = bt.t[slot + 1] - bt.t[slot];
   const double* yi = bt.y + (size_t)slot * CS_NY;
@@ -2796,8 +2797,8 @@ __device__ void cs_condense_big(const CsBatch& bt, int slot, double* slab, doubl
         if (r < pr && c < kb) P[r * CS_PLD + c] = x[s][c];
     }
     if (w == 0) {
-      moved[lane] = src;
-      moved[32 + lane] = dst;
+      moved[lane] = (short)src;
+      moved[32 + lane] = (short)dst;
     }
     __syncthreads();
     // panel rows 0..kb-1 (U11, multipliers below its diagonal) back to the slab

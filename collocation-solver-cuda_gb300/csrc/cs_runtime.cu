@@ -577,7 +577,7 @@ extern "C" int cs_module_load(const cs_module_desc* d, cs_module** out) {
     const long long nb = 16, ncol1 = s1 + M->nrhs, ldg = ((ncol1 + 3) / 4) * 4, nfg = d->ny + d->nz + d->np;
     const long long ws_jf = (long long)d->m * rb * nfg + (long long)rb * M->nrhs + d->m * d->m + d->m;
     const long long ws_cond = (long long)s1 * ldg + ws_jf + (d->precision ? (ws_jf + 1) / 2 : 0ll);
-    const long long sm_cond = (long long)s1 * (nb + 1) + nb * ldg + (long long)d->m * rb + d->m * d->m + d->ny + s1 + 16 + 4 * nb;
+    const long long sm_cond = (long long)s1 * (nb + 1) + nb * ldg + (long long)d->m * rb + d->m * d->m + d->ny + s1 + 16 + nb;
     const long long qsz = (long long)qld * qc, tsz = (long long)tld * (nt + 1);
     const long long drsz = (long long)(d->ny + d->np) * (2 * d->ny + d->np);
     // CS_SM_QR(ld) in cs_kernels.cuh

@@ -57,7 +57,8 @@ class CompiledProblem:
 
     layout: 0 automatic, 1 shared-memory kernels only, 2 the large-system
     kernels (global-memory slab per CTA; chosen automatically when a stage
-    system or a BABD block does not fit in shared memory).
+    system or a BABD block does not fit in shared memory, and for the BABD
+    solve from ny = 28 on).
     precision: "fp64" (default), "tf32" or "bf16": the large-system
     condensation on the tensor cores (an inexact Newton Jacobian; residual,
     line search, mesh error and BABD solve stay FP64); "tf32-tree" /

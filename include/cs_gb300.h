@@ -72,7 +72,8 @@ typedef struct cs_module_desc {
                                shared memory (fails if they do not fit);
                                2: large-system kernels (global-memory slab per
                                CTA, blocked LU), chosen automatically when the
-                               blocks do not fit in shared memory */
+                               blocks do not fit in shared memory, and for the
+                               BABD solve from ny = 28 on */
   int precision;            /* large-system condensation: 0 FP64; 1 TF32,
                                2 BF16 tensor cores with FP32 storage and
                                accumulation (an inexact Newton Jacobian: the
@@ -231,8 +232,9 @@ int cs_stage_remesh(cs_batch* bt, const double* res, int* N_new);
  * Outputs dy ((n+1) x ny) and dp (np) in device memory; *singular (host, may
  * be NULL) is set when the top system was singular (dy_0, dy_n, dp are then 0,
  * as the reference's LinAlgError fallback).  1 <= ny <= 32, 0 <= np <= 32.
- * Allocates its scratch (about 8 (2 ny (2ny+np+1) + ny (3ny+np+1)) bytes per
- * interval) for the duration of the call; ordered on `stream` (a
+ * Takes its scratch (at most about 8 (2 ny (2ny+np+1) + ny (3ny+np+1)) bytes
+ * per interval) from a memory pool of the library (which keeps up to 256 MB
+ * between calls) for the duration of the call; ordered on `stream` (a
  * cudaStream_t or NULL) and returns after it has finished.
  * Replaces: partition_factorization_parallel, construct_babd_mshoot,
  * qr_decomposition, backward_substitution, recover_babd_solution and
@@ -390,9 +392,10 @@ int cs_last_error(char* buf, size_t len);
 int cs_time_condense(cs_batch* bt, int reps, double* ms);
 
 /* Launch-shape tuner of the condensation (the per-(m, ny) tile shape):
- * times every candidate on the batch's current intervals -- 4, 8, 16 or 32
- * lanes per interval x 1..8 warps per CTA for shared-memory stage systems,
- * 128 or 256 threads per CTA for the large-system kernel -- and makes the
+ * times every candidate on the batch's current intervals -- 1, 2 or 4 warps per
+ * CTA where the condensation runs in registers, 4, 8, 16 or 32 lanes per
+ * interval x 1..8 warps per CTA for other shared-memory stage systems, the grid
+ * of the large-system kernel -- and makes the
  * fastest the module's shape for all its batches.  No reference
  * counterpart. */
 typedef struct cs_tune_result {
