@@ -349,7 +349,7 @@ class Workload:
 # about a million intervals of each m-group (working set far above L2:
 # dram__bytes_read.sum + dram__bytes_write.sum ÷ intervals,
 # profiles/k_condense_vdp_batch3072_mix.md)
-TRAFFIC_PER_INTERVAL_NCU = {3: 1000.4, 4: 1240.4, 5: 1474.0}
+TRAFFIC_PER_INTERVAL_NCU = {3: 1000.3, 4: 1243.6, 5: 1491.5}
 
 
 def flops_per_interval(m, ny=4, nz=1, npe=0):
@@ -441,7 +441,7 @@ def _roofline(groups, fp64_peak):
             "traffic": (traffic / len(groups)) if traffic == traffic else None,
             "traffic_note": "DRAM bytes per launch (average over the m-groups): bytes per interval measured by ncu "
                             "for each m on a launch of ~1M intervals (profiles/k_condense_vdp_batch3072_mix.md: "
-                            "1000 / 1240 / 1474 B for m = 3 / 4 / 5, 92-94 % of the algorithmic bytes) times the "
+                            "1000 / 1244 / 1491 B for m = 3 / 4 / 5, 92-95 % of the algorithmic bytes) times the "
                             "intervals of this launch; algorithmic bytes per interval are in flops_note",
             "peak_source": "DFMA microbenchmark (cs_measure_fp64_peak) in this run, best of repeated runs over "
                            "about a second with the SM clock sampled meanwhile (peak_measurement); FP64 is absent "
