@@ -2521,11 +2521,13 @@ __device__ __forceinline__ unsigned cs_dyn_smem_bytes() {
 }
 
 // the launch gives this CTA (last: the last CTA of its cluster, so that a
-// cluster decides as one) a slab of at least `slab` doubles and `sm`
-// doubles of shared memory; otherwise count a configuration error and do
-// nothing (the host reports it)
-__device__ __forceinline__ bool cs_big_ok(const CsBatch& bt, long long slab, long long sm, int last) {
-  const bool ok = blockDim.x <= 256 && (blockDim.x & 31) == 0 && (long long)cs_dyn_smem_bytes() >= sm * 8 &&
+// cluster decides as one) a slab of at least `slab` doubles, `sm` doubles of
+// shared memory and the `threads` its work is dealt out by (0: any whole
+// warps up to 256); otherwise count a configuration error and do nothing
+// (the host reports it)
+__device__ __forceinline__ bool cs_big_ok(const CsBatch& bt, long long slab, long long sm, int last, int threads) {
+  const bool ok = (threads ? (int)blockDim.x == threads : blockDim.x <= 256 && (blockDim.x & 31) == 0) &&
+                  (long long)cs_dyn_smem_bytes() >= sm * 8 &&
                   (slab == 0 || (bt.wsp != nullptr && last < bt.wsp_ctas && bt.wsp_stride >= slab));
   if (!ok && threadIdx.x == 0) atomicAdd(&bt.counters[7], 1ull);
   return ok;
@@ -3359,9 +3361,9 @@ __device__ bool cs_condense_tc(const CsBatch& bt, int slot, double* slab, unsign
 extern "C" __global__ void __launch_bounds__(256, 2) k_condense(CsBatch bt) {
   extern __shared__ __align__(128) double smem[];
 #if CS_PREC == 0
-  if (!cs_big_ok(bt, CS_WS_COND, CS_SM_COND, blockIdx.x)) return;
+  if (!cs_big_ok(bt, CS_WS_COND, CS_SM_COND, blockIdx.x, CS_COND_TB)) return;
 #else
-  if (!cs_big_ok(bt, CS_WS_COND, CS_TC_SMD, blockIdx.x)) return;
+  if (!cs_big_ok(bt, CS_WS_COND, CS_TC_SMD, blockIdx.x, 0)) return;
   // the CTA's tensor-memory accumulator and MMA barrier, for all its intervals
   unsigned char* smb = reinterpret_cast<unsigned char*>(smem);
   unsigned long long* mb = reinterpret_cast<unsigned long long*>(smb + CS_TC_MISC);
@@ -3902,12 +3904,12 @@ extern "C" __global__ void __launch_bounds__(CS_TREE_TB, CS_NY <= 256 ? 512 / CS
   const int G = (int)cs_cluster_size(), rank = (int)cs_cluster_rank();
   const int first = (int)blockIdx.x - rank;  // the cluster's first CTA owns its slab
 #if CS_PREC_TREE == 0
-  if (!cs_big_ok(bt, CS_WS_TREE, CS_SM_TREE, first + G - 1)) return;
+  if (!cs_big_ok(bt, CS_WS_TREE, CS_SM_TREE, first + G - 1, CS_TREE_TB)) return;
   double* Q = bt.wsp + (size_t)first * bt.wsp_stride;
   double* sh = smem;
   double* Rd = bt.wsp + (size_t)blockIdx.x * bt.wsp_stride + CS_QSZ;
 #else
-  if (!cs_big_ok(bt, CS_WS_TREE_LP, CS_SM_TREE_LP, blockIdx.x)) return;
+  if (!cs_big_ok(bt, CS_WS_TREE_LP, CS_SM_TREE_LP, blockIdx.x, 0)) return;
   float* Q = reinterpret_cast<float*>(CS_Q_SMEM_LP ? smem : bt.wsp + (size_t)blockIdx.x * bt.wsp_stride);
   double* sh = CS_Q_SMEM_LP ? smem + CS_QSZ_LP : smem;
 #endif
@@ -3951,7 +3953,7 @@ extern "C" __global__ void __launch_bounds__(CS_TREE_TB, CS_NY <= 256 ? 512 / CS
 __device__ void cs_top_big(const CsBatch& bt, double* smem, const double* dyk, const double* dpk) {
   const int G = (int)cs_cluster_size(), rank = (int)cs_cluster_rank();
   const int first = (int)blockIdx.x - rank;
-  if (!cs_big_ok(bt, CS_WS_TOP, CS_SM_TOP, first + G - 1)) return;
+  if (!cs_big_ok(bt, CS_WS_TOP, CS_SM_TOP, first + G - 1, 256)) return;
   double* top = bt.wsp + (size_t)first * bt.wsp_stride;
   double* Dr = top + CS_TSZ;
   double* Rd = bt.wsp + (size_t)blockIdx.x * bt.wsp_stride + CS_TSZ + CS_DRSZ;

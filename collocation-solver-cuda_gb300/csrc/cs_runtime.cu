@@ -1155,7 +1155,8 @@ static int run_condense(cs_batch* bt, CsBatchDev& v) {
 }
 
 // large-system kernels count a launch that gave them too little shared
-// memory or slab in counters[7] and skip their work
+// memory or slab, or another CTA size than theirs, in counters[7] and skip
+// their work
 static int check_config(cs_batch* bt) {
   if (!bt->M->big) return CS_OK;
   unsigned long long c7 = 0;
@@ -1163,7 +1164,7 @@ static int check_config(cs_batch* bt) {
   CS_CUDA(cudaStreamSynchronize(bt->stream));
   if (c7 != 0)
     return set_err(CS_ERR_STATE,
-                   "large-system kernel launched without its shared memory or slab, or a tensor-core MMA timed out");
+                   "large-system kernel launched without its shared memory, slab or CTA size, or a tensor-core MMA timed out");
   return CS_OK;
 }
 
@@ -2341,13 +2342,23 @@ extern "C" int cs_autotune_condense(cs_batch* bt, int reps, cs_tune_result* out)
       }
     }
   } else {
-    // one CTA per interval: CTA size; the grid stays within the CTAs that
-    // have a slab in this batch
-    for (int block = 128; block <= 256; block *= 2) {
+    // one CTA per interval; the grid stays within the CTAs that have a slab in
+    // this batch.  FP64: the work is dealt out by a CTA size fixed at compile
+    // time (CS_COND_TB), so the CTAs per SM are all there is to choose; reduced
+    // precision: the CTA size
+    if (!M->prec) {
       int per_sm = 0;
-      CS_CU(g_drv.occupancy(&per_sm, M->f_condense, block, M->condense_smem));
-      const int grid = std::min(M->sms * std::max(1, per_sm), M->big_ctas);
-      cands.push_back({M->f_condense, 0, block, grid, M->condense_smem});
+      CS_CU(g_drv.occupancy(&per_sm, M->f_condense, M->condense_block, M->condense_smem));
+      for (int p = 1; p <= per_sm && M->sms * p <= M->big_ctas; ++p)
+        if (M->sms * p != M->condense_grid)
+          cands.push_back({M->f_condense, 0, M->condense_block, M->sms * p, M->condense_smem});
+    } else {
+      for (int block = 128; block <= 256; block *= 2) {
+        int per_sm = 0;
+        CS_CU(g_drv.occupancy(&per_sm, M->f_condense, block, M->condense_smem));
+        const int grid = std::min(M->sms * std::max(1, per_sm), M->big_ctas);
+        cands.push_back({M->f_condense, 0, block, grid, M->condense_smem});
+      }
     }
   }
   cudaEvent_t e0, e1;

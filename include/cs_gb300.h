@@ -394,9 +394,9 @@ int cs_time_condense(cs_batch* bt, int reps, double* ms);
 /* Launch-shape tuner of the condensation (the per-(m, ny) tile shape):
  * times every candidate on the batch's current intervals -- 1, 2 or 4 warps per
  * CTA where the condensation runs in registers, 4, 8, 16 or 32 lanes per
- * interval x 1..8 warps per CTA for other shared-memory stage systems, the grid
- * of the large-system kernel -- and makes the
- * fastest the module's shape for all its batches.  No reference
+ * interval x 1..8 warps per CTA for other shared-memory stage systems, the CTAs
+ * per SM (FP64) or the CTA size (reduced precision) of the large-system kernel --
+ * and makes the fastest the module's shape for all its batches.  No reference
  * counterpart. */
 typedef struct cs_tune_result {
   int lanes;          /* lanes per interval, 0: one CTA per interval */
