@@ -48,9 +48,11 @@ __device__ __forceinline__ double cs_rsqrt(double x) {
 // leading entry x0: H column = g e_0 (the sign rule of
 // matrix_factorization_cuda.py:37-54), v_0 = x0 - g, v the column below, and
 // t = 2 / |v|^2 = 1 / (ss + |x0 g|) = r^2 / (1 + |x0| r), r = ss^(-1/2).  False
-// when |v|^2 / 2 is below `least` (the bits of a positive double; eps / 2 by
-// default: nothing to eliminate).  A square root and two divisions before: with
-// few merges in flight their latency (about 600 cycles each) was a third of a
+// when |v|^2 / 2 is a number below `least` (the bits of a positive double; eps / 2
+// by default: nothing to eliminate).  A column with a NaN reflects, and so hands it
+// on to every column: skipped, what it holds below the diagonal would be dropped
+// and the solution would come out finite.  A square root and two divisions before:
+// with few merges in flight their latency (about 600 cycles each) was a third of a
 // merge.  Its users form the products p_c = column . column c of the untouched
 // columns first: p of the column itself is ss, and v . column c = p_c - g times
 // the leading entry of column c, so one pass over the rows serves both.
@@ -62,9 +64,10 @@ __device__ __forceinline__ bool cs_reflector(double ss, double x0, double* g, do
   *g = gg;
   *v0 = x0 - gg;
   *t = (r * r) * cs_rcp(q);
-  // |v|^2 / 2 = ss q, as integers (false for NaN)
-  const long long b = __double_as_longlong(ss * q);
-  return b >= least && b <= 0x7ff0000000000000ll;
+  // |v|^2 / 2 = ss q, as integers: a NaN is above every number.  A zero ss makes
+  // q infinite and the product a NaN: tested by itself
+  const long long b = __double_as_longlong(ss * q) & 0x7fffffffffffffffll;
+  return b >= least && (__double_as_longlong(ss) << 1) != 0;
 }
 
 #endif  // CS_FP64_CUH
