@@ -2196,11 +2196,19 @@ extern "C" __global__ void __launch_bounds__(256) k_backsub_level(CsBatch bt, in
 // them, and each level is otherwise a round trip to L2.  Levels below go
 // through k_tree_level / k_backsub_level before and after this launch.
 // Measured (4 levels and the top system of 333 instances): 84 -> 64 us.
+// The top system's space is what cs_top_warp takes: the boundary rows where its
+// columns are in registers, else the whole system (CS_TLD x (CS_NT + 1)), which
+// grows with the parameters and comes with the launch.
 #define CS_UROWS 16
 extern "C" __global__ void __launch_bounds__(128) k_upper(CsBatch bt, int l_first) {
+#if CS_TOP_LANES
+  __shared__ double top[(CS_NY + CS_NP) * (2 * CS_NY + CS_NP + 1)];
+#else
+  extern __shared__ double smem[];
+  double* top = smem;
+#endif
   __shared__ double rows[2][CS_UROWS * CS_ROWSZ];
   __shared__ double recs[CS_UROWS * CS_TREESZ];  // of the node at position e (units of 2^l_lo)
-  __shared__ double top[(CS_NY + CS_NP) * (2 * CS_NY + CS_NP + 1)];
   __shared__ double nodes[(CS_UROWS + 1) * CS_NY];
   const int groups = blockDim.x / CS_TL, grp = threadIdx.x / CS_TL, c = threadIdx.x & (CS_TL - 1);
   const int njac = bt.nlist[1];

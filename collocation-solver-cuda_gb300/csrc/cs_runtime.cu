@@ -405,8 +405,9 @@ struct cs_module {
   CUfunction f_refine_res = nullptr, f_top_refine = nullptr, f_refine_add = nullptr;
   size_t babd_cta_smem;
   // k_upper (upper tree levels, top and their back substitution, CTA per
-  // instance): 0 when the block rows are too large for lane merges
+  // instance): not when the block rows are too large for lane merges
   bool upper = false;
+  size_t upper_smem = 0;
   int upper_grid = 0;
   // one wave of resident CTAs: grids of the grid-stride kernels k_residual and
   // k_tree_level (small block rows), so that launches with little work do not
@@ -664,8 +665,14 @@ extern "C" int cs_module_load(const cs_module_desc* d, cs_module** out) {
     M->top_wpc = (int)std::max<size_t>(1, std::min<size_t>(4, (size_t)smem_optin / top_per));
     M->babd_cta_smem = top_per + (size_t)8 * qld * qc * sizeof(double);
     M->top_smem = top_per * M->top_wpc;
-    // CS_TREE_THREAD && CS_QC <= 32 in cs_kernels.cuh (lane merges)
-    if (2 * M->ny * qc <= 128 && qc <= 32) M->upper = true;
+    // CS_TREE_THREAD && CS_QC <= 32 in cs_kernels.cuh (lane merges); beside its
+    // static rows, records and nodes k_upper holds the top system in the launch's
+    // shared memory unless its columns are in registers (CS_TOP_LANES)
+    if (2 * M->ny * qc <= 128 && qc <= 32) {
+      M->upper_smem = 2 * M->ny + M->np <= 16 ? 0 : top_per;
+      const size_t fixed = ((size_t)16 * (2 * M->rowsz + M->treesz) + 17 * M->ny) * sizeof(double);
+      M->upper = fixed + M->upper_smem <= (size_t)smem_optin;
+    }
   }
 
   std::string src = build_source(d, M->big_cond, M->big_tree, M->prec, M->big_tree ? M->prec_tree : 0, smem_optin);
@@ -790,8 +797,10 @@ extern "C" int cs_module_load(const cs_module_desc* d, cs_module** out) {
     }
   }
   if (M->upper) {
+    if (M->upper_smem > 16 * 1024)  // (the static arrays take up to 24 of the 48 KB)
+      CS_CU(g_drv.funcSetAttribute(M->f_upper, CU_FUNC_ATTRIBUTE_MAX_DYNAMIC_SHARED_SIZE_BYTES, (int)M->upper_smem));
     int pu = 0;
-    CS_CU(g_drv.occupancy(&pu, M->f_upper, 128, 0));
+    CS_CU(g_drv.occupancy(&pu, M->f_upper, 128, M->upper_smem));
     M->upper_grid = M->sms * std::max(1, std::min(pu, 16));
   }
   if (M->babd_cta_smem > (size_t)smem_optin) M->babd_cta_smem = 0;  // per-level kernels only
@@ -1276,7 +1285,7 @@ static int run_direction(cs_batch* bt, CsBatchDev& v, int nlvl) {
   if (M->upper && bt->opts.babd_path != 2) {
     int lo = l_lo;
     void* a[] = {&v, &lo};
-    CS_TRY(launch_k(bt, M->f_upper, capped_inst(bt, (unsigned)std::min(M->upper_grid, bt->B)), 128, 0, a, 1));
+    CS_TRY(launch_k(bt, M->f_upper, capped_inst(bt, (unsigned)std::min(M->upper_grid, bt->B)), 128, M->upper_smem, a, 1));
   } else {
     void* a[] = {&v};
     if (M->big_tree) CS_TRY(launch_cluster(bt, M->f_top, gtop, 256, M->top_smem, ctop, a, 1));
