@@ -270,23 +270,28 @@ extern "C" int cs_format_double(double v, char* out) {
     if (e_ != cudaSuccess) return cs_internal_set_error(CS_ERR_CUDA, (std::string(what) + ": " + cudaGetErrorString(e_)).c_str()); \
   } while (0)
 
+static void scratch_drop(CsTextScratch* s, int i) {
+  cudaFree(s->p[i]);
+  s->p[i] = nullptr;
+  s->bytes[i] = 0;
+}
+
 void cs_text_scratch_free(CsTextScratch* s) {
-  for (int i = 0; i < 2; ++i) {
-    cudaFree(s->p[i]);
-    s->p[i] = nullptr;
-    s->bytes[i] = 0;
-  }
+  for (int i = 0; i < 2; ++i) scratch_drop(s, i);
 }
 
 static int scratch_grow(CsTextScratch* s, int i, size_t bytes) {
   if (s->bytes[i] >= bytes) return CS_OK;
-  cudaFree(s->p[i]);
-  s->p[i] = nullptr;
-  s->bytes[i] = 0;
+  scratch_drop(s, i);
   CS_TRYC(cudaMalloc(&s->p[i], bytes), "cs_format_solutions: scratch");
   s->bytes[i] = bytes;
   return CS_OK;
 }
+
+// The text buffer stays with the batch up to this size (as the library's pool
+// keeps); a larger one goes back to the device before the call returns.  Below it
+// an allocation would cost as much as the writing: 62 MB of text take 0.9 ms.
+static const size_t kTextKeep = 256ull << 20;
 
 int cs_text_files(const CsTextArgs& a, char* out, long long cap, long long* offsets) {
   std::vector<long long> pre(a.B + 1);
@@ -339,5 +344,6 @@ int cs_text_files(const CsTextArgs& a, char* out, long long cap, long long* offs
   CS_TRYC(cudaGetLastError(), "k_text_write");
   CS_TRYC(cudaMemcpyAsync(out, a.scratch->p[1], (size_t)total, cudaMemcpyDeviceToHost, st), "cs_format_solutions: text to host");
   CS_TRYC(cudaStreamSynchronize(st), "cs_format_solutions");
+  if (a.scratch->bytes[1] > kTextKeep) scratch_drop(a.scratch, 1);
   return CS_OK;
 }

@@ -280,6 +280,8 @@ int cs_tc_update(int precision, int M, int N, int K, const float* A, int lda, co
  * the values cs_get_solution returns.  offsets (B + 1 entries) are always
  * filled: file b is out[offsets[b] .. offsets[b+1]).  out = NULL only sizes
  * the files; a cap below offsets[B] fails with CS_ERR_INVALID.
+ * The device copy of the text stays with the batch for the next call up to 256 MB
+ * (until cs_batch_free); a larger one is freed before the call returns.
  * Replaces: the per-value Python writer (BVPDAEReadWriteData.py:337-364)
  * called once per solution. */
 int cs_format_solutions(cs_batch* bt, char* out, long long cap, long long* offsets);
