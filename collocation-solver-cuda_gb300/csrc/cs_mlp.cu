@@ -690,6 +690,19 @@ static int mlp_buf(cs_mlp::Buf& b, size_t bytes) {
   return CS_OK;
 }
 
+// At the end of a call (its stream idle): copies of the caller's arrays stay for
+// the next call up to this size each (four thousand samples of 322 outputs are
+// 5 MB), larger ones go back to the device.
+constexpr size_t kMlpKeep = 256ull << 20;
+static void mlp_give_back(cs_mlp* M) {
+  for (cs_mlp::Buf* b : {&M->in_x, &M->in_y, &M->in_perm, &M->out_y})
+    if (b->bytes > kMlpKeep) {
+      cudaFree(b->p);
+      b->p = nullptr;
+      b->bytes = 0;
+    }
+}
+
 static void net_describe(cs_mlp* M) {
   NetDesc& d = M->net;
   memset(&d, 0, sizeof(d));
@@ -1055,11 +1068,11 @@ extern "C" int cs_mlp_gradient(cs_mlp* M, const float* X, const float* Y, int n,
     rc = mlp_forward(M, n);
     if (rc == CS_OK) rc = mlp_backward(M, n, loss);
   }
-  if (rc == CS_OK && grad) {
-    cudaError_t e = cudaMemcpyAsync(grad, M->g, M->nparam * sizeof(float), cudaMemcpyDeviceToHost, M->st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(M->st);
-    if (e != cudaSuccess) rc = cs_internal_set_error(CS_ERR_CUDA, cudaGetErrorString(e));
-  }
+  cudaError_t e = cudaSuccess;
+  if (rc == CS_OK && grad) e = cudaMemcpyAsync(grad, M->g, M->nparam * sizeof(float), cudaMemcpyDeviceToHost, M->st);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(M->st);
+  if (rc == CS_OK && e != cudaSuccess) rc = cs_internal_set_error(CS_ERR_CUDA, cudaGetErrorString(e));
+  mlp_give_back(M);
   return rc;
 }
 
@@ -1125,6 +1138,7 @@ extern "C" int cs_mlp_train(cs_mlp* M, const float* X, const float* Y, int n, in
   }
   cudaError_t e = cudaStreamSynchronize(M->st);
   if (rc == CS_OK && e != cudaSuccess) rc = cs_internal_set_error(CS_ERR_CUDA, cudaGetErrorString(e));
+  mlp_give_back(M);
   if (final_loss) *final_loss = last;
   return rc;
 }
@@ -1195,5 +1209,6 @@ extern "C" int cs_mlp_predict(cs_mlp* M, const float* X, int n, float* Y) {
   }
   cudaError_t e = cudaStreamSynchronize(M->st);
   if (rc == CS_OK && e != cudaSuccess) rc = cs_internal_set_error(CS_ERR_CUDA, cudaGetErrorString(e));
+  mlp_give_back(M);
   return rc;
 }

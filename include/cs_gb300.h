@@ -322,8 +322,10 @@ void cs_pinned_free(void* p);
  * depth linear layers n_in -> width -> ... -> width -> n_out, GELU between
  * them; FP32 master weights, BF16 operands with FP32 accumulation on the
  * tensor cores, MSE loss on normalised outputs, Adam.  Host arrays are
- * row-major float32 (one row per sample).  No counterpart in the reference
- * (its Newton starts from the OCP file's constant estimates). */
+ * row-major float32 (one row per sample).  Device copies of the host arrays of a
+ * call stay with the network for the next call, up to 256 MB each, until
+ * cs_mlp_free; larger ones are freed before the call returns.  No counterpart in
+ * the reference (its Newton starts from the OCP file's constant estimates). */
 typedef struct cs_mlp cs_mlp;
 int cs_mlp_create(int n_in, int width, int depth, int n_out, unsigned long long seed, cs_mlp** out);
 void cs_mlp_free(cs_mlp* mlp);

@@ -1,5 +1,6 @@
 """Device memory that calls keep: the solution writer's text buffer stays with its
-batch up to 256 MB and goes back to the device above."""
+batch up to 256 MB and goes back to the device above, and so do the network's
+copies of a call's host arrays."""
 import numpy as np
 import pytest
 
@@ -43,3 +44,19 @@ def test_large_text_buffers_go_back_to_the_device():
     text, _ = large.solution_text()
     assert len(text) > 256 * MB
     assert before - free_memory() < 64 * MB
+
+
+def test_large_training_sets_go_back_to_the_device():
+    cs = pkg()
+    rng = np.random.default_rng(0)
+    X, Y = rng.random((66000, 4), dtype=np.float32), rng.random((66000, 1100), dtype=np.float32)  # Y: 290 MB
+    net = cs.warmstart.Mlp(4, 1100, width=32, depth=3, seed=1)
+    net.fit_normalization(X[:2048], Y[:2048])
+    net.train(X[:2048], Y[:2048], epochs=1, batch=1024, lr=1e-3)  # training buffers, kernels
+    first = net.predict(X[:2048])
+    before = free_memory()
+    net.train(X, Y, epochs=1, batch=1024, lr=0.0)
+    assert before - free_memory() < 64 * MB
+    whole = net.predict(X)  # 65,536 rows at a time: 288 MB of output
+    assert before - free_memory() < 64 * MB
+    np.testing.assert_array_equal(whole[:2048], first)
