@@ -47,26 +47,33 @@ __device__ __forceinline__ double cs_rsqrt(double x) {
 // Householder reflector H = I - t v v^T of a column with sum of squares ss and
 // leading entry x0: H column = g e_0 (the sign rule of
 // matrix_factorization_cuda.py:37-54), v_0 = x0 - g, v the column below, and
-// t = 2 / |v|^2 = 1 / (ss + |x0 g|) = r^2 / (1 + |x0| r), r = ss^(-1/2).  False
-// when |v|^2 / 2 is a number below `least` (the bits of a positive double; eps / 2
-// by default: nothing to eliminate).  A column with a NaN reflects, and so hands it
-// on to every column: skipped, what it holds below the diagonal would be dropped
-// and the solution would come out finite.  A square root and two divisions before:
-// with few merges in flight their latency (about 600 cycles each) was a third of a
-// merge.  Its users form the products p_c = column . column c of the untouched
-// columns first: p of the column itself is ss, and v . column c = p_c - g times
-// the leading entry of column c, so one pass over the rows serves both.
+// t = 2 / |v|^2 = 1 / (ss + |x0 g|).  False when |v|^2 / 2 is a number below
+// `least` (the bits of a positive double; eps / 2 by default: nothing to
+// eliminate).  A column with a NaN reflects, and so hands it on to every column:
+// skipped, what it holds below the diagonal would be dropped and the solution
+// would come out finite.
+//
+// a = ss r, r = ss^(-1/2), is sqrt(ss) to 2.5 of 2^-53; g takes a Newton step
+// from it, a + (ss - a^2) r / 2, as exact as a rounded square root and beside the
+// chain a, |v|^2 / 2, t (t to 3.3 of 2^-53).  A square root and two divisions
+// before: with few merges in flight their latency (about 600 cycles each) was a
+// third of a merge.  Its users form the products p_c = column . column c of the
+// untouched columns first: p of the column itself is ss, and v . column c = p_c -
+// g times the leading entry of column c, so one pass over the rows serves both.
 __device__ __forceinline__ bool cs_reflector(double ss, double x0, double* g, double* v0, double* t,
                                              long long least = 0x3ca0000000000000ll) {
   const double r = cs_rsqrt(ss);
-  const double a = ss * r, q = fma(fabs(x0), r, 1.0);
-  const double gg = (__double2hiint(x0) >= 0) ? cs_neg(a) : a;
+  const double a = ss * r;
+  const double s = fma(fabs(x0), a, ss);  // |v|^2 / 2
+  // (r / 2 by its exponent; where r is 0, infinite or a NaN so is a a NaN)
+  const double w = fma(fma(-a, a, ss), __hiloint2double(__double2hiint(r) - (1 << 20), __double2loint(r)), a);
+  const double gg = (__double2hiint(x0) >= 0) ? cs_neg(w) : w;
   *g = gg;
   *v0 = x0 - gg;
-  *t = (r * r) * cs_rcp(q);
-  // |v|^2 / 2 = ss q, as integers: a NaN is above every number.  A zero ss makes
-  // q infinite and the product a NaN: tested by itself
-  const long long b = __double_as_longlong(ss * q) & 0x7fffffffffffffffll;
+  *t = cs_rcp(s);
+  // as integers: a NaN is above every number.  A zero ss makes r infinite and s
+  // a NaN: tested by itself
+  const long long b = __double_as_longlong(s) & 0x7fffffffffffffffll;
   return b >= least && (__double_as_longlong(ss) << 1) != 0;
 }
 

@@ -6,8 +6,10 @@ Bounds (in units of the last place of the result, from the series):
   cs_rcp       final rounding 1/2, cut-off e^3 < 2^-67 of the value < 2^-14 ulp: 0.51
   cs_rsqrt     final rounding 1/2, rounding of x r in h up to 1/2, cut-off
                5/16 h^3 < 2^-63 of the value < 2^-10 ulp: 1.01
-  g            cs_rsqrt's 3/2 of 2^-53 relative and the product's rounding: 2.5 of
-               2^-53 relative, at most 2.51 ulp
+  g            final rounding of the Newton step, whose cut-off (2.5 2^-53)^2 / 2 and
+               rounding of a residual of 5 2^-53 are far below: 0.51
+  t            half of a's 2.5 of 2^-53 (|x0| a is at most half of |v|^2 / 2), two
+               roundings of 1: 3.25 of 2^-53 relative, and the cut-offs: 3.3
 """
 import ctypes
 import os
@@ -125,12 +127,10 @@ def test_reflector_of_ordinary_columns(lib, seed_error):
             ss, x0 = float(np.dot(c, c)), float(c[0])
             assert lib.reflector(ss, x0, out, LEAST_BABD)
             g = Decimal(ss).sqrt() * (-1 if x0 >= 0 else 1)
-            assert ulps(out[0], g) <= Decimal("2.51")
+            assert ulps(out[0], g) <= Decimal("0.51")
             assert out[1] == x0 - out[0]
-            # t |v|^2 / 2 = 1 at the exact square root: r^2 (4 of 2^-53 relative), the
-            # reciprocal and q (4 together)
             t = 1 / (Decimal(ss) + abs(Decimal(x0) * g))
-            assert abs(Decimal(out[2]) / t - 1) <= 8 * Decimal(2)**-53
+            assert abs(Decimal(out[2]) / t - 1) <= Decimal("3.3") * Decimal(2)**-53
     lib.set_seed_error(0)
 
 
