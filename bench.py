@@ -361,6 +361,20 @@ def flops_per_interval(m, ny=4, nz=1, npe=0):
     return 2.0 / 3.0 * s ** 3 + 2.0 * s * s * r
 
 
+def executed_flops_per_interval(m, ny, nz, npe):
+    """FP64 flops the condensation executes per interval, r right-hand sides.
+    Small stage systems (the kernel's own rule): LU of the sy = (m-1) ny rows
+    left when the algebraic unknowns have been eliminated stage by stage, the
+    right-hand sides' substitutions, and filling both (2 sy^2 + 2 sy r ny); the
+    eliminated unknowns' own few operations are not counted.  Others: LU of the
+    stage system without its stage-0 block (s1 = (m-1)(ny+nz) rows), the
+    substitutions, and the stage-0 coupling of the right-hand sides (2 s1 r ny)."""
+    r, sy = ny + npe + 1, (m - 1) * ny
+    small = sy <= 28 and nz * (nz + r) <= 80
+    s1 = sy if small else (m - 1) * (ny + nz)
+    return 2.0 / 3.0 * s1 ** 3 + 2.0 * s1 * s1 * r + 2.0 * s1 * r * ny + (2.0 * s1 * s1 if small else 0.0)
+
+
 def bytes_per_interval(m, ny=4, nz=1, npe=0):
     """Algorithmic HBM bytes of condensing one interval: read t, y_i, y_{i+1},
     y', z~; write X = W^-1 [J V f_a] and the block row [A C H b]."""
@@ -422,7 +436,7 @@ def _sum_over_ranks(dist, x):
 def _roofline(groups, fp64_peak):
     """Condensation of every interval of each group, timed alone with CUDA
     events on the batch's stream (one launch per group)."""
-    flops = cbytes = cms = traffic = 0.0
+    flops = done = cbytes = cms = traffic = 0.0
     n_all = 0
     for m, bt in groups:
         bt.reset()
@@ -430,12 +444,13 @@ def _roofline(groups, fp64_peak):
         n_int = bt.sizes()[1] - bt.B
         cp = bt.cp
         flops += n_int * flops_per_interval(m, cp.ny, cp.nz, cp.np_eff)
+        done += n_int * executed_flops_per_interval(m, cp.ny, cp.nz, cp.np_eff)
         cbytes += n_int * bytes_per_interval(m, cp.ny, cp.nz, cp.np_eff)
         cms += ms
         n_all += n_int
         # measured for the Van der Pol family only (ny = 4)
         traffic += (TRAFFIC_PER_INTERVAL_NCU.get(m, float("nan")) if cp.ny == 4 else float("nan")) * n_int
-    achieved = flops / (cms * 1e-3) / 1e12
+    achieved = done / (cms * 1e-3) / 1e12
     return {"bound": "fp64", "kernel": "k_condense", "achieved": achieved, "peak": fp64_peak, "unit": "TFLOP/s",
             "frac": achieved / fp64_peak if fp64_peak else None,
             "traffic": (traffic / len(groups)) if traffic == traffic else None,
@@ -446,10 +461,11 @@ def _roofline(groups, fp64_peak):
             "peak_source": "DFMA microbenchmark (cs_measure_fp64_peak) in this run, best of repeated runs over "
                            "about a second with the SM clock sampled meanwhile (peak_measurement); FP64 is absent "
                            "from MEASURED_PEAKS.json",
-            "flops_per_launch": flops / len(groups), "ms_per_launch": cms / len(groups),
-            "flops_note": "contract flops per interval (2/3)s^3 + 2 s^2 r, s = m(ny+nz), r = ny+np_eff+1; "
-                          "the kernel executes about half of them (stage 0 and the algebraic unknowns are "
-                          "eliminated apart), so frac can exceed 1; "
+            "flops_per_launch": done / len(groups), "ms_per_launch": cms / len(groups),
+            "contract_tflops": flops / (cms * 1e-3) / 1e12, "contract_flops_per_launch": flops / len(groups),
+            "flops_note": "achieved and frac: the flops the kernel executes, (2/3)sy^3 + 2 sy^2 (r + 1) + 2 sy r ny "
+                          "per interval with sy = (m-1)ny, r = ny+np_eff+1 where the algebraic unknowns are "
+                          "eliminated apart; contract: (2/3)s^3 + 2 s^2 r, s = m(ny+nz), of the whole stage system; "
                           "algorithmic bytes 8(2 + 2ny + m(ny+nz) + r s + ny(2ny+np_eff+1)) per interval",
             "hbm_gbs": cbytes / (cms * 1e-3) / 1e9}
 
@@ -729,16 +745,6 @@ def pendulum_problem(cs, K):
     return cs.workloads.pendulum_chain_problem(K)
 
 
-def executed_flops_per_interval(m, ny, nz, npe):
-    """FP64 flops the structured condensation executes per interval: LU of
-    the stage system without its stage-0 block (s1 = (m-1)(ny+nz) rows) with
-    r right-hand sides, their back substitution, and the stage-0 coupling of
-    the right-hand sides (2 s1 r ny)."""
-    s1 = (m - 1) * (ny + nz)
-    r = ny + npe + 1
-    return 2.0 / 3.0 * s1 ** 3 + 2.0 * s1 * s1 * r + 2.0 * s1 * r * ny
-
-
 def _cpu_pendulum(cs, pr, m, slice_intervals=256):
     """The oracle (numpy, BLAS threads on all host cores) on one residual and
     one Newton step of the first `slice_intervals` intervals of the mesh;
@@ -885,15 +891,16 @@ def run_pendulum(args, cs, rank, world, local_rank):
         except (OSError, KeyError, ValueError):
             peak = 1900.0
         bound = "tensor"
-    roof = {"bound": bound, "kernel": "k_condense", "achieved": fc * n_int / (ms * 1e-3) / 1e12, "peak": peak,
-            "unit": "TFLOP/s", "frac": fc * n_int / (ms * 1e-3) / 1e12 / peak, "traffic": None,
-            "ms_per_launch": ms, "flops_per_launch": fc * n_int,
-            "executed_tflops": fe * n_int / (ms * 1e-3) / 1e12,
-            "executed_frac": fe * n_int / (ms * 1e-3) / 1e12 / fp64_peak,
-            "flops_note": "achieved: contract flops (2/3)s^3 + 2 s^2 r per interval, s = m(ny+nz) = %d, r = %d; "
-                          "executed: (2/3)s1^3 + 2 s1^2 r + 2 s1 r ny with s1 = (m-1)(ny+nz) = %d (the stage-0 "
-                          "block is eliminated directly); peak of measured FP64 (DFMA microbenchmark, this run)"
-                          % (m * (cp.ny + cp.nz), cp.ny + cp.np_eff + 1, (m - 1) * (cp.ny + cp.nz))}
+    roof = {"bound": bound, "kernel": "k_condense", "achieved": fe * n_int / (ms * 1e-3) / 1e12, "peak": peak,
+            "unit": "TFLOP/s", "frac": fe * n_int / (ms * 1e-3) / 1e12 / peak, "traffic": None,
+            "ms_per_launch": ms, "flops_per_launch": fe * n_int,
+            "contract_tflops": fc * n_int / (ms * 1e-3) / 1e12,
+            "frac_of_fp64": fe * n_int / (ms * 1e-3) / 1e12 / fp64_peak,
+            "flops_note": "achieved and frac: executed flops, (2/3)s1^3 + 2 s1^2 r + 2 s1 r ny per interval with "
+                          "s1 = (m-1)(ny+nz) = %d (the stage-0 block is eliminated directly), r = %d; contract: "
+                          "(2/3)s^3 + 2 s^2 r, s = m(ny+nz) = %d; frac_of_fp64: of the measured FP64 peak (DFMA "
+                          "microbenchmark, this run)"
+                          % ((m - 1) * (cp.ny + cp.nz), cp.ny + cp.np_eff + 1, m * (cp.ny + cp.nz))}
     # reduced precision: max-abs difference from the FP64 solve of the same problem
     err = None
     if args.precision != "fp64":
