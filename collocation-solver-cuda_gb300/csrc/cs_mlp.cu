@@ -632,6 +632,7 @@ struct cs_mlp {
   int* didx = nullptr;
   // fused kernels (every layer at most kNetDim wide)
   bool fused = false;
+  int sms = 1;        // of the network's device
   NetDesc net;
   __nv_bfloat16* pack = nullptr;
   bool stale = true;  // the packed weights are older than w
@@ -755,8 +756,7 @@ static size_t net_smem(const NetDesc& d, int mt) { return (size_t)2 * 16 * mt * 
 // (64 rows per CTA: 59 / 61 / 61).  Training holds pre-activations and
 // gradients back and keeps 16 warps throughout: <2, 16, 2, 4> above one block
 // per SM.
-constexpr int kSms = 152;
-static int net_rows(const NetDesc& d, int n) { return (n <= 16 * kSms || net_smem(d, 2) > 200 * 1024) ? 16 : 32; }
+static int net_rows(const NetDesc& d, int n, int sms) { return (n <= 16 * sms || net_smem(d, 2) > 200 * 1024) ? 16 : 32; }
 
 static void net_free(cs_mlp* M) {
   cudaFree(M->xk);
@@ -818,8 +818,8 @@ static int net_predict(cs_mlp* M, const float* dX, int n, float* dY, cudaStream_
   g.pack = M->pack;
   g.n = n;
   g.out = dY;
-  if (net_rows(M->net, n) == 16) return net_launch<1, 16, 2, 8, false>(M, g, st);
-  if (n <= 32 * kSms) return net_launch<2, 16, 2, 8, false>(M, g, st);
+  if (net_rows(M->net, n, M->sms) == 16) return net_launch<1, 16, 2, 8, false>(M, g, st);
+  if (n <= 32 * M->sms) return net_launch<2, 16, 2, 8, false>(M, g, st);
   return net_launch<2, 8, 4, 4, false>(M, g, st);
 }
 
@@ -846,7 +846,7 @@ static int net_step(cs_mlp* M, const float* dX, const float* dY, const int* idx,
   g.dk = M->dk;
   g.pre = M->kpre;
   g.bsum = M->bsum;
-  const int rows = net_rows(d, n);
+  const int rows = net_rows(d, n, M->sms);
   rc = rows == 16 ? net_launch<1, 16, 2, 8, true>(M, g, M->st) : net_launch<2, 16, 2, 4, true>(M, g, M->st);
   if (rc != CS_OK) return rc;
   int tiles = 0;
@@ -901,7 +901,9 @@ extern "C" int cs_mlp_create(int n_in, int width, int depth, int n_out, unsigned
   // weights
   const size_t pb = (off * sizeof(float) + 255) / 256 * 256, nb = (nrm.size() * sizeof(float) + 255) / 256 * 256;
   const size_t kb = M->fused ? net_pack_elems(M->net) * sizeof(__nv_bfloat16) : 0;
-  if (cudaStreamCreateWithFlags(&M->st, cudaStreamNonBlocking) != cudaSuccess ||
+  int dev = 0;
+  if (cudaStreamCreateWithFlags(&M->st, cudaStreamNonBlocking) != cudaSuccess || cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&M->sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
       cudaMalloc(&M->block, 4 * pb + nb + 256 + kb) != cudaSuccess ||
       (kb && cudaMemsetAsync(M->block + 4 * pb + nb + 256, 0, kb, M->st) != cudaSuccess)) {
     cs_mlp_free(M);
