@@ -258,7 +258,7 @@ __global__ void kb_back(BabdDims d, int l, const double* tree, const double* dp,
 // Blocks up to 16 x 16: subtrees.  A merge is a chain of ny reflectors, a few
 // microseconds whatever the machine, and a system of a thousand rows has eleven
 // levels of them: launches and round trips to L2 between the levels cost as
-// much again.  So a CTA takes kRows consecutive rows through four levels in
+// much again.  So a CTA takes kRows = 8 consecutive rows through three levels in
 // shared memory (kb_sub; the first reads the caller's arrays), until one CTA
 // holds what is left (kb_root: last levels, top system, first levels down), and
 // the back substitution comes down the same chunks (kb_down).  A merge is one
